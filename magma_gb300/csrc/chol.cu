@@ -160,19 +160,19 @@ __global__ void __launch_bounds__(256)
 chol_solve_kernel(int n, int nrhs, T **dA_array, int lda, T **dB_array, int ldb)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(16) Diag<T> sD;
     T *sB = reinterpret_cast<T *>(smem_raw);
-    const int mat = blockIdx.y, tid = threadIdx.x;
+    const int mat = blockIdx.y, tid = threadIdx.x, ldx = solve_ldx<T>(n);
     const int c0 = blockIdx.x * CHOL_NR, nr = min(CHOL_NR, nrhs - c0);
     T *B = dB_array[mat] + (size_t)c0 * ldb;
     for (int e = tid; e < CHOL_NR * n; e += blockDim.x) {
         const int c = e / n, i = e % n;
-        sB[e] = c < nr ? B[i + (size_t)c * ldb] : T(0);
+        sB[c * ldx + i] = c < nr ? B[i + (size_t)c * ldb] : T(0);
     }
-    __syncthreads();
-    chol_solve_smem<T, CHOL_NR>(n, dA_array[mat], lda, sB);
+    chol_solve_smem<T, solve_cg<T, CHOL_NR>()>(n, dA_array[mat], lda, sB, ldx, nr, sD);
     for (int e = tid; e < nr * n; e += blockDim.x) {
         const int c = e / n, i = e % n;
-        B[i + (size_t)c * ldb] = sB[c * n + i];
+        B[i + (size_t)c * ldb] = sB[c * ldx + i];
     }
 }
 
@@ -180,7 +180,7 @@ template <typename T>
 magma_int_t chol_solve(int n, int nrhs, T **dA, int lda, T **dB, int ldb, int batch,
                        magma_queue_t q)
 {
-    const size_t smem = (size_t)CHOL_NR * n * sizeof(T);
+    const size_t smem = (size_t)CHOL_NR * solve_ldx<T>(n) * sizeof(T);
     static size_t dyn_cache[MLU_MAX_DEVICES];
     const size_t dyn_max = mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(chol_solve_kernel<T>); });
     if (smem > dyn_max) return MAGMA_ERR_NOT_SUPPORTED;

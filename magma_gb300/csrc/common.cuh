@@ -64,11 +64,58 @@ template <> struct Prec<float> {
     __device__ static inline float fma_(float a, float b, float c) { return fmaf(a, b, c); }
 };
 
+// The FP64 division as a call: where it is the rare path (below), its inlined
+// start would be issued, predicated off, on the common one.
+static __device__ __noinline__ double div_call(double a, double b) { return a / b; }
+
+// Correctly rounded 1/x off the FP64 pipe, which is what most FP64 kernels here
+// wait for: a warp's division takes 86 cycles of an SM's FP64 pipe (5.4 FMAs)
+// and 364 cycles of latency, these integer instructions 27 cycles of issue and
+// 275 of latency.  A single-precision approximation y0 of 1/m (m: the
+// significand), one cubic Newton step y0 (1 + r + r^2), r = 1 - m y0, in 64-bit
+// fixed point (off by less than one unit of the result), then the exact
+// remainder 2^105 - q m decides the last bit; 2^106 = (2q + 1) m has no solution
+// but for powers of two, so there are no ties.  Zero, subnormal, infinite and
+// NaN operands, and those whose reciprocal is subnormal, take the division.
+__device__ __forceinline__ double recip(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned e = (hi >> 20) & 0x7ffu;
+    if (e - 1u > 2043u) return div_call(1.0, x);
+    const unsigned mh = (hi & 0xfffffu) | 0x100000u;                  // m = mh:lo, 53 bits
+    const unsigned d1 = __funnelshift_l(lo, mh, 11), d0 = lo << 11;   // m << 11
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(0x3f800000u | ((d1 >> 8) & 0x7fffffu))));
+    const unsigned yb = max(__float_as_uint(y), 0x3f000000u);
+    const unsigned y0 = yb >= 0x3f800000u ? 0xffffffffu : (yb << 8) | 0x80000000u;   // 2^32 y, y in [1/2, 1]
+    // r = 1 - m y0, scaled by 2^64: |r| < 2^-21
+    const unsigned long long p1 = (unsigned long long)d1 * y0, p0 = (unsigned long long)d0 * y0;
+    const long long r = (long long)(0ull - ((p1 << 1) + (p0 >> 31)));
+    const int rh = (int)(r >> 12);
+    const long long s = r + (long long)((unsigned)__mulhi(rh, rh) >> 8);
+    // y1 = y0 (1 + s), scaled by 2^63, and rounded to the 53 bits of the result
+    const long long t = (long long)(int)(s >> 32) * (long long)(unsigned long long)y0 +
+                        (long long)__umulhi((unsigned)s, y0);
+    const unsigned long long y1 = ((unsigned long long)y0 << 31) + (unsigned long long)(t >> 1);
+    unsigned long long q = (y1 + 512ull) >> 10;
+    const long long m = (long long)(((unsigned long long)mh << 32) | lo);
+    const long long rem2 = 2 * (long long)(0ull - q * (unsigned long long)m);
+    q += rem2 > m ? 1ull : 0ull;
+    q -= rem2 < -m ? 1ull : 0ull;
+    // q's leading bit (bit 52, or 53 for a power of two) carries into the exponent
+    const unsigned long long b = q + ((unsigned long long)(2044u - e) << 52);
+    return __longlong_as_double((long long)(b | ((unsigned long long)(hi & 0x80000000u) << 32)));
+}
+__device__ __forceinline__ float recip(float x) { return 1.f / x; }
+
 // x scaled by the reciprocal r of d, or divided by d when d is subnormal
 // (LAPACK dgetf2's sfmin rule).
-template <typename T>
-__device__ __forceinline__ T rscale(T x, T d, T r) {
-    return Prec<T>::normal_or_special(d) ? x * r : x / d;
+__device__ __forceinline__ double rscale(double x, double d, double r) {
+    if (Prec<double>::normal_or_special(d)) return x * r;
+    return div_call(x, d);
+}
+__device__ __forceinline__ float rscale(float x, float d, float r) {
+    return Prec<float>::normal_or_special(d) ? x * r : x / d;
 }
 
 // ---------------------------------------------------------------------------

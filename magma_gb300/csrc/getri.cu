@@ -25,30 +25,28 @@ __global__ void __launch_bounds__(GETRI_THREADS)
 getri_kernel(int n, T **dA_array, int ldda, int **ipiv_array, T **dInv_array, int lddia)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sB = reinterpret_cast<T *>(smem_raw);                              // [NR][n]
-    int *s_perm = reinterpret_cast<int *>(sB + (size_t)GETRI_NR * n);     // [n]
+    __shared__ __align__(16) Diag<T> sD;
+    __shared__ int s_col[GETRI_NR];                                       // output columns
+    T *sB = reinterpret_cast<T *>(smem_raw);                              // [NR][ldx]
+    const int ldx = solve_ldx<T>(n);
     const int mat = blockIdx.y, tid = threadIdx.x;
     const int j0 = blockIdx.x * GETRI_NR;
     const int nr = min(GETRI_NR, n - j0);
     const int *ipiv = ipiv_array[mat];
-    for (int i = tid; i < n; i += blockDim.x) s_perm[i] = i;
     for (int e = tid; e < GETRI_NR * n; e += blockDim.x) {
         const int c = e / n, i = e % n;
-        sB[e] = (c < nr && i == j0 + c) ? T(1) : T(0);
+        sB[c * ldx + i] = (c < nr && i == j0 + c) ? T(1) : T(0);
     }
-    __syncthreads();
-    if (tid == 0) {
-        for (int k = 0; k < n; k++) {
-            const int p = ipiv[k] - 1;
-            if (p != k) { const int t = s_perm[k]; s_perm[k] = s_perm[p]; s_perm[p] = t; }
-        }
+    if (tid < nr) {
+        int tau[1] = {j0 + tid};
+        resolve_rows(tau, ipiv, n);
+        s_col[tid] = tau[0];
     }
-    __syncthreads();
-    solve_smem<T, false, GETRI_NR>(n, dA_array[mat], ldda, nullptr, sB, nr);
+    solve_smem<T, false, solve_cg<T, GETRI_NR>()>(n, dA_array[mat], ldda, sB, ldx, nr, sD);
     T *Inv = dInv_array[mat];
     for (int e = tid; e < nr * n; e += blockDim.x) {
         const int c = e / n, i = e % n;
-        Inv[i + (size_t)s_perm[j0 + c] * lddia] = sB[c * n + i];
+        Inv[i + (size_t)s_col[c] * lddia] = sB[c * ldx + i];
     }
 }
 
@@ -67,10 +65,13 @@ static magma_int_t getri_run(const char *name, magma_int_t n, T **dA_array, magm
         return info;
     }
     if (n == 0 || batchCount == 0) return 0;
-    const size_t smem = (size_t)GETRI_NR * n * sizeof(T) + (size_t)n * sizeof(int);
+    const size_t smem = (size_t)GETRI_NR * solve_ldx<T>(n) * sizeof(T);
     static size_t dyn_cache[MLU_MAX_DEVICES];
     const size_t dyn_max = mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(getri_kernel<T>); });
-    if (smem > dyn_max) return MAGMA_ERR_NOT_SUPPORTED;
+    // the largest order: the right-hand sides and one int per row in shared memory
+    const size_t limit = dyn_max + GETRI_NR * sizeof(int) + (sizeof(T) == 4 ? 128 + 32 * 3 * sizeof(T) : 0);
+    if ((size_t)GETRI_NR * n * sizeof(T) + (size_t)n * sizeof(int) > limit || smem > dyn_max)
+        return MAGMA_ERR_NOT_SUPPORTED;
     const int threads = min(GETRI_THREADS, max(64, (n + 31) / 32 * 32));
     cudaStream_t s = queue->stream;
     for (int b0 = 0; b0 < batchCount; b0 += MLU_MAX_GRID_Y) {

@@ -280,7 +280,8 @@ ir_solve_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, double
                 double tol, const double *rowscale, const double *colscale)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float *sB = reinterpret_cast<float *>(smem_raw);
+    float *sB = reinterpret_cast<float *>(smem_raw);   // [NR][ldx]
+    __shared__ __align__(16) Diag<float> sD;
     __shared__ int s_go;
     const int mat = blockIdx.y, tid = threadIdx.x;
     const int n = sh.N(mat), nrhs = sh.NR(mat), lddx = sh.LDX(mat);
@@ -306,13 +307,13 @@ ir_solve_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, double
         for (int e = tid; e < 2 * IR_NRHS_MAX + 2; e += blockDim.x) nx[e] = 0ull;
     }
     const int c0 = blockIdx.x * NR;
-    const int nr = min(NR, nrhs - c0);
+    const int nr = min(NR, nrhs - c0), ldx = solve_ldx<float>(n);
     const double *Rm = R + ((size_t)mat * sh.nrhs + c0) * sh.n;
     const int *pm = SPD ? nullptr : perm + (size_t)mat * sh.n;
     if (SPD) {
         for (int e = tid; e < NR * n; e += blockDim.x) {
             const int c = e / n, i = e % n;
-            sB[c * n + i] = __double2float_rn(c < nr ? Rm[i + (size_t)c * sh.n] : 0.0);
+            sB[c * ldx + i] = __double2float_rn(c < nr ? Rm[i + (size_t)c * sh.n] : 0.0);
         }
     } else if (!TRANS) {
         // row interchanges applied while loading: sB[i] = R[perm[i]]
@@ -320,22 +321,20 @@ ir_solve_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, double
             const int c = e / n, i = e % n;
             const int p = pm[i];
             const double rv = c < nr ? Rm[p + (size_t)c * sh.n] : 0.0;
-            sB[c * n + i] = __double2float_rn(rowscale ? rv * rowscale[(size_t)mat * sh.n + p] : rv);
+            sB[c * ldx + i] = __double2float_rn(rowscale ? rv * rowscale[(size_t)mat * sh.n + p] : rv);
         }
     } else {
         for (int e = tid; e < NR * n; e += blockDim.x) {
             const int c = e / n, i = e % n;
-            sB[c * n + i] = __double2float_rn(c < nr ? Rm[i + (size_t)c * sh.n] : 0.0);
+            sB[c * ldx + i] = __double2float_rn(c < nr ? Rm[i + (size_t)c * sh.n] : 0.0);
         }
     }
-    __syncthreads();
-    if (SPD) chol_solve_smem<float, NR>(n, dAs_array[mat], ldas, sB);
-    else solve_smem<float, TRANS, NR, true>(n, dAs_array[mat], ldas, nullptr, sB, nr);
-    __syncthreads();
+    if (SPD) chol_solve_smem<float, NR>(n, dAs_array[mat], ldas, sB, ldx, nr, sD);
+    else solve_smem<float, TRANS, NR>(n, dAs_array[mat], ldas, sB, ldx, nr, sD);
     double *X = dX_array[mat] + (size_t)c0 * lddx;
     for (int e = tid; e < nr * n; e += blockDim.x) {
         const int c = e / n, i = e % n;
-        const double d = (double)sB[c * n + i];
+        const double d = (double)sB[c * ldx + i];
         // A^T: the interchanges undone on the way out, x[perm[i]] += w[i]
         const int r = (TRANS && !SPD) ? pm[i] : i;
         X[r + (size_t)c * lddx] = X[r + (size_t)c * lddx] +
@@ -574,14 +573,14 @@ template <int NR>
 __host__ __device__ inline size_t gm_smem_bytes(int n)
 {
     const int m = n < GM_INNER_MAX ? n : GM_INNER_MAX;
-    return sizeof(float) * ((size_t)2 * NR * n + (size_t)NR * (m + 1) * m + (size_t)NR * (3 * m + 1));
+    return sizeof(float) * ((size_t)NR * (solve_ldx<float>(n) + n) + (size_t)NR * (m + 1) * m + (size_t)NR * (3 * m + 1));
 }
 
 // check (as ir_solve_kernel) + GMRES correction X += d for the nrhs <= NR
 // right-hand sides of one matrix.  V: per right-hand side GM_INNER_MAX+1 FP32
 // vectors of n.
 template <int NR>
-__global__ void __launch_bounds__(GM_THREADS)
+__global__ void __launch_bounds__(GM_THREADS, 2)
 gm_correction_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, const float *A32,
                      double **dX_array, const double *R, unsigned long long *stats, int *iter,
                      int *inner_total, int it, double tol, const double *rowscale,
@@ -590,13 +589,15 @@ gm_correction_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, c
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float s_red[GM_WARPS][NR], s_sum[NR];
     __shared__ double s_red64[GM_WARPS][NR], s_sum64[NR];
+    __shared__ __align__(16) Diag<float> sD;
     __shared__ int s_go, s_act[NR], s_k[NR], s_any;
     const int mat = blockIdx.y, tid = threadIdx.x;
     const int n = sh.N(mat), nrhs = sh.NR(mat), lddx = sh.LDX(mat);
     if (n == 0 || nrhs == 0) return;
     const int m = min(GM_INNER_MAX, n);
-    float *sB = reinterpret_cast<float *>(smem_raw);   // [NR][n]: preconditioner input / output
-    float *sW = sB + NR * n;                           // [NR][n]: Arnoldi vector
+    const int ldx = solve_ldx<float>(n);
+    float *sB = reinterpret_cast<float *>(smem_raw);   // [NR][ldx]: preconditioner input / output
+    float *sW = sB + NR * ldx;                           // [NR][n]: Arnoldi vector
     float *sH = sW + NR * n;                           // [NR][m+1][m]: Hessenberg matrices
     float *sCs = sH + NR * (m + 1) * m;                // [NR][m]
     float *sSn = sCs + NR * m;                         // [NR][m]
@@ -685,13 +686,11 @@ gm_correction_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, c
                 x = V(c, i)[p];
                 if (rsc) x *= (float)rsc[p];
             }
-            sB[c * n + q] = x;
+            sB[c * ldx + q] = x;
         }
-        __syncthreads();
-        solve_smem<float, false, NR>(n, LU, ldas, nullptr, sB, nr);
-        __syncthreads();
+        solve_smem<float, false, NR>(n, LU, ldas, sB, ldx, nr, sD);
         if (csc) {
-            for (int e = tid; e < NR * n; e += GM_THREADS) sB[e] *= (float)csc[e % n];
+            for (int e = tid; e < NR * n; e += GM_THREADS) sB[(e / n) * ldx + e % n] *= (float)csc[e % n];
             __syncthreads();
         }
         // w = A z
@@ -704,7 +703,7 @@ gm_correction_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, c
             for (int j = 0; j < n; j++) {
                 const float a = Ar[(size_t)j * ldas];
 #pragma unroll
-                for (int c = 0; c < NR; c++) acc[c] = fmaf(a, sB[c * n + j], acc[c]);
+                for (int c = 0; c < NR; c++) acc[c] = fmaf(a, sB[c * ldx + j], acc[c]);
             }
 #pragma unroll
             for (int c = 0; c < NR; c++) sW[c * n + r] = acc[c];
@@ -788,16 +787,14 @@ gm_correction_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, c
             for (int j = 0; j < s_k[c]; j++) t = fmaf(sRs[c * (m + 1) + j], V(c, j)[p], t);
             if (rsc) t *= (float)rsc[p];
         }
-        sB[c * n + q] = t;
+        sB[c * ldx + q] = t;
     }
-    __syncthreads();
-    solve_smem<float, false, NR>(n, LU, ldas, nullptr, sB, nr);
-    __syncthreads();
+    solve_smem<float, false, NR>(n, LU, ldas, sB, ldx, nr, sD);
     double *X = dX_array[mat];
     for (int e = tid; e < nr * n; e += GM_THREADS) {
         const int c = e / n, q = e % n;
         if (s_k[c] == 0) continue;
-        const double d = (double)sB[c * n + q];
+        const double d = (double)sB[c * ldx + q];
         X[q + (size_t)c * lddx] += beta[c] * (csc ? d * csc[q] : d);
     }
     if (tid == 0) {
@@ -981,7 +978,7 @@ static void correction_solve(const IrShape &sh, float **As_array, int ldas, cons
                              const double *csc, int batch, cudaStream_t s, bool spd = false)
 {
     const int snr = sh.nrhs <= 4 ? 4 : IR_SOLVE_NR;   // right-hand sides per CTA
-    const size_t ssmem = (size_t)snr * sh.n * sizeof(float);
+    const size_t ssmem = (size_t)snr * solve_ldx<float>(sh.n) * sizeof(float);
     const dim3 grid(mlu_ceildiv(sh.nrhs, snr), batch);
     if (spd) {
         if (snr == 4)
@@ -1017,6 +1014,7 @@ static void correction_solve(const IrShape &sh, float **As_array, int ldas, cons
 static int residual_nr(int nrhs) { return nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : nrhs <= 4 ? 4 : nrhs <= 8 ? 8 : 16; }
 static int solve_nr(int nrhs) { return nrhs <= 4 ? 4 : IR_SOLVE_NR; }
 constexpr size_t IR_RESIDUAL_SMEM_MAX = 200 * 1024;   // X rows of the residual, in shared memory
+constexpr size_t IR_SOLVE_SMEM_MAX = 222960;          // right-hand sides of the correction solve
 
 static size_t solve_dyn_max();
 
@@ -1027,7 +1025,7 @@ static size_t solve_dyn_max();
 static bool ir_fits(const char *name, int n, int nrhs)
 {
     const size_t rb = (size_t)residual_nr(nrhs) * sizeof(double), sb = (size_t)solve_nr(nrhs) * sizeof(float);
-    const size_t smax = solve_dyn_max();
+    const size_t smax = min(solve_dyn_max(), IR_SOLVE_SMEM_MAX);
     if ((size_t)n * rb <= IR_RESIDUAL_SMEM_MAX && (size_t)n * sb <= smax) return true;
     const size_t nmax = min(IR_RESIDUAL_SMEM_MAX / rb, smax / sb);
     fprintf(stderr, "%s: order n=%d with nrhs=%d does not fit the refinement's shared-memory right-hand "

@@ -32,6 +32,8 @@
 #include "lu_core.cuh"
 #include "solve_core.cuh"
 
+#include <type_traits>
+
 namespace mlu {
 
 constexpr int PANEL_THREADS = PANEL_REGS_THREADS;
@@ -838,40 +840,43 @@ template magma_int_t blocked_getrf_vbatched<float>(const int *, const int *, con
                                                    float **, int **, int *, int, magma_queue_t);
 
 // ---------------------------------------------------------------------------
-// Blocked solves.  One CTA per (matrix, group of SOLVE_NR right-hand sides);
-// the right-hand sides live in shared memory.  Triangular blocks of 32 are
-// solved by warp 0 with shuffles, the rows below/above are then updated by
-// all threads; every element receives its updates in the oracle's order.
+// Blocked solves.  One CTA per (matrix, group of nc right-hand sides) runs the
+// two triangular sweeps of solve_core.cuh on them in shared memory.
 
 constexpr int SOLVE_THREADS = 256;
-constexpr int SOLVE_NR = 8;
+constexpr int SOLVE_NC = 8;                // right-hand sides per CTA, at most
 
-// One CTA per (matrix, group of NR right-hand sides); NR is 4 or 8 so that a
-// call with few right-hand sides does not spend FMAs on padding columns.
-template <typename T, bool TRANS, int NR>
-__global__ void __launch_bounds__(SOLVE_THREADS)
-getrs_kernel(int n, int nrhs, T **dA_array, int ldda, int **ipiv_array, T **dB_array, int lddb)
+// CG: right-hand sides per update task (FP32: nc is a multiple of it).
+// `stage_piv`: the pivots fit in shared memory behind the right-hand sides.
+template <typename T, bool TRANS, int CG>
+__global__ void __launch_bounds__(SOLVE_THREADS, sizeof(T) == 8 ? 2 : 3)
+getrs_kernel(int n, int nrhs, T **dA_array, int ldda, int **ipiv_array, T **dB_array, int lddb, int nc,
+             int stage_piv)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sB = reinterpret_cast<T *>(smem_raw);   // [NR][n]
-    const int tid = threadIdx.x;
+    __shared__ __align__(16) Diag<T> sD;
+    T *sB = reinterpret_cast<T *>(smem_raw);   // [nc][ldx]
+    const int ldx = solve_ldx<T>(n);
+    int *s_piv = stage_piv ? reinterpret_cast<int *>(sB + (size_t)nc * ldx) : nullptr;
     const int mat = blockIdx.y;
-    const int c0 = blockIdx.x * NR;
-    const int nr = min(NR, nrhs - c0);
+    const int c0 = blockIdx.x * nc;
+    const int nr = min(nc, nrhs - c0);
     const T *A = dA_array[mat];
     const int *ipiv = ipiv_array ? ipiv_array[mat] : nullptr;   // null: no interchanges
     T *B = dB_array[mat] + (size_t)c0 * lddb;
+    move_rhs<T, false>(n, TRANS ? nullptr : ipiv, s_piv, B, lddb, sB, ldx, nr, nc);
+    solve_smem<T, TRANS, CG>(n, A, ldda, sB, ldx, nr, sD);
+    move_rhs<T, true>(n, TRANS ? ipiv : nullptr, s_piv, B, lddb, sB, ldx, nr, nc);
+}
 
-    for (int e = tid; e < NR * n; e += blockDim.x) {
-        const int c = e / n, i = e % n;
-        sB[c * n + i] = c < nr ? B[i + (size_t)c * lddb] : T(0);
-    }
-    __syncthreads();
-    solve_smem<T, TRANS, NR>(n, A, ldda, ipiv, sB, nr);
-    for (int e = tid; e < nr * n; e += blockDim.x) {
-        const int c = e / n, i = e % n;
-        B[i + (size_t)c * lddb] = sB[c * n + i];
-    }
+template <typename T, bool TRANS, int CG>
+static void launch_getrs(dim3 grid, int threads, size_t smem, cudaStream_t s, int n, int nrhs, T **A, int ldda,
+                         int **P, T **B, int lddb, int nc, int stage_piv)
+{
+    static size_t dyn_cache[MLU_MAX_DEVICES];
+    mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(getrs_kernel<T, TRANS, CG>); });
+    MLU_LAUNCH(mlu::KC_GETRS, s, getrs_kernel<T, TRANS, CG><<<grid, threads, smem, s>>>(
+        n, nrhs, A, ldda, P, B, lddb, nc, stage_piv));
 }
 
 template <typename T>
@@ -879,38 +884,38 @@ magma_int_t blocked_getrs(bool trans, int n, int nrhs, T **dA, int ldda, int **i
                           int lddb, int batch, magma_queue_t q)
 {
     if (batch <= 0 || n == 0 || nrhs == 0) return MAGMA_SUCCESS;
-    const int nr = nrhs <= 4 ? 4 : SOLVE_NR;
-    const size_t smem = (size_t)nr * n * sizeof(T);
-    static size_t dyn_cache[2][2][MLU_MAX_DEVICES];
-    size_t *cache = dyn_cache[trans][nr == 4];
-    const size_t dm = mlu_device_cached(cache, [&] {
-        if (trans) return nr == 4 ? mlu_allow_dynamic_smem(getrs_kernel<T, true, 4>)
-                                  : mlu_allow_dynamic_smem(getrs_kernel<T, true, SOLVE_NR>);
-        return nr == 4 ? mlu_allow_dynamic_smem(getrs_kernel<T, false, 4>)
-                       : mlu_allow_dynamic_smem(getrs_kernel<T, false, SOLVE_NR>);
-    });
-    if (smem > dm) return MAGMA_ERR_NOT_SUPPORTED;
-    // one thread per row up to 256 (at least two warps: warp 0 solves the
-    // diagonal blocks while the others wait)
-    const int threads = min(SOLVE_THREADS, max(64, (n + 31) / 32 * 32));
+    static size_t dyn_cache[MLU_MAX_DEVICES];
+    const size_t dm = mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(getrs_kernel<T, false, 1>); });
+    // the largest order: four (or, with more right-hand sides, eight) columns in shared memory
+    if ((size_t)(nrhs <= 4 ? 4 : SOLVE_NC) * n * sizeof(T) > dm) return MAGMA_ERR_NOT_SUPPORTED;
+    // Right-hand sides per CTA: eight, fewer while that leaves SMs without a CTA
+    // (the sweeps of different right-hand sides do not wait for one another) or
+    // while they do not fit.  FP32: as many as one update task takes.
+    const size_t col = (size_t)solve_ldx<T>(n) * sizeof(T);
+    int nc = sizeof(T) == 4 ? (nrhs == 1 ? 1 : nrhs <= 4 ? 4 : SOLVE_NC) : min(nrhs, SOLVE_NC);
+    while (nc > 1 && ((long long)batch * mlu_ceildiv(nrhs, nc) < mlu_sm_count() || nc * col > dm))
+        nc = sizeof(T) == 4 ? (nc == 8 ? 4 : 1) : (nc + 1) / 2;
+    const bool stage_piv = ipiv != nullptr && nc * col + (size_t)n * sizeof(int) <= dm;
+    const size_t smem = nc * col + (stage_piv ? (size_t)n * sizeof(int) : 0);
+    // FP64: four warps use the whole FP64 pipe, eight when an SM has one CTA; FP32:
+    // one thread per row up to 256
+    const int threads = sizeof(T) == 8 ? ((long long)batch * mlu_ceildiv(nrhs, nc) >= 2 * mlu_sm_count() ? 128 : 256)
+                                       : min(SOLVE_THREADS, max(64, (n + 31) / 32 * 32));
     cudaStream_t s = q->stream;
     for (int b0 = 0; b0 < batch; b0 += MLU_MAX_GRID_Y) {
         const int nb = min(batch - b0, (int)MLU_MAX_GRID_Y);
-        const dim3 grid((nrhs + nr - 1) / nr, nb);
+        const dim3 grid((nrhs + nc - 1) / nc, nb);
         T **A = dA + b0, **B = dB + b0;
         int **P = ipiv ? ipiv + b0 : nullptr;
-        if (trans && nr == 4)
-            MLU_LAUNCH(mlu::KC_GETRS, s, getrs_kernel<T, true, 4><<<grid, threads, smem, s>>>(
-                n, nrhs, A, ldda, P, B, lddb));
-        else if (trans)
-            MLU_LAUNCH(mlu::KC_GETRS, s, getrs_kernel<T, true, SOLVE_NR><<<grid, threads, smem, s>>>(
-                n, nrhs, A, ldda, P, B, lddb));
-        else if (nr == 4)
-            MLU_LAUNCH(mlu::KC_GETRS, s, getrs_kernel<T, false, 4><<<grid, threads, smem, s>>>(
-                n, nrhs, A, ldda, P, B, lddb));
-        else
-            MLU_LAUNCH(mlu::KC_GETRS, s, getrs_kernel<T, false, SOLVE_NR><<<grid, threads, smem, s>>>(
-                n, nrhs, A, ldda, P, B, lddb));
+        auto go = [&](auto cg) {
+            constexpr int CG = decltype(cg)::value;
+            if (trans) launch_getrs<T, true, CG>(grid, threads, smem, s, n, nrhs, A, ldda, P, B, lddb, nc, stage_piv);
+            else launch_getrs<T, false, CG>(grid, threads, smem, s, n, nrhs, A, ldda, P, B, lddb, nc, stage_piv);
+        };
+        if (nc == 1) go(std::integral_constant<int, 1>{});
+        else if constexpr (sizeof(T) == 8) go(std::integral_constant<int, 2>{});
+        else if (nc == 4) go(std::integral_constant<int, 4>{});
+        else go(std::integral_constant<int, 8>{});
     }
     MLU_CHECK_LAUNCH();
     return MAGMA_SUCCESS;

@@ -33,6 +33,7 @@ namespace mlu {
 constexpr int VB_THREADS = PANEL_REGS_THREADS;   // the register panel runs on all threads
 constexpr int VB_BINS = 1024;
 constexpr int VB_NR = 16;                  // right-hand sides per solve pass
+constexpr int VB_SOLVE_NR = 8;             // right-hand sides per CTA of the separate solve
 constexpr size_t VB_SMEM_CAP = 220 * 1024;
 
 // Per-size-bin tuning of the persistent kernel: panel width and trailing-update
@@ -119,6 +120,7 @@ vb_lu_kernel(const int *m_arr, const int *n_arr, const int *nrhs_arr, T **dA_arr
              VbTune tune)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(16) Diag<T> sD;
     __shared__ int s_item, s_ipiv[PANEL_NB], s_row[2 * PANEL_NB], s_src[2 * PANEL_NB], s_cnt;
     const int tid = threadIdx.x, warp = tid >> 5;
     T *sT = reinterpret_cast<T *>(smem);
@@ -176,50 +178,39 @@ vb_lu_kernel(const int *m_arr, const int *n_arr, const int *nrhs_arr, T **dA_arr
         }
         if (tid == 0) info_array[k] = info;
         if (nrhs > 0 && m == n && n > 0) {
+            const int ldx = solve_ldx<T>(n);
             for (int c0 = 0; c0 < nrhs; c0 += VB_NR) {
                 const int nr = min(VB_NR, nrhs - c0);
                 T *Bc = B + (size_t)c0 * ldb;
                 __syncthreads();
-                for (int e = tid; e < VB_NR * n; e += VB_THREADS) {
-                    const int c = e / n, i = e % n;
-                    sT[c * n + i] = c < nr ? Bc[i + (size_t)c * ldb] : T(0);
-                }
-                __syncthreads();
-                solve_smem<T, false, VB_NR>(n, A, lda, nullptr, sT, nr);
-                for (int e = tid; e < nr * n; e += VB_THREADS) {
-                    const int c = e / n, i = e % n;
-                    Bc[i + (size_t)c * ldb] = sT[c * n + i];
-                }
+                move_rhs<T, false>(n, nullptr, nullptr, Bc, ldb, sT, ldx, nr, VB_NR);
+                solve_smem<T, false, solve_cg<T, VB_NR>(), 16>(n, A, lda, sT, ldx, nr, sD);
+                move_rhs<T, true>(n, nullptr, nullptr, Bc, ldb, sT, ldx, nr, VB_NR);
             }
         }
     }
 }
 
-// Solve with existing factors, one CTA per (matrix, group of VB_NR columns).
+// Solve with existing factors, one CTA per (matrix, group of VB_SOLVE_NR columns).
 template <typename T, bool TRANS>
-__global__ void __launch_bounds__(VB_THREADS)
+__global__ void __launch_bounds__(VB_THREADS, 2)
 vb_getrs_kernel(const int *n_arr, const int *nrhs_arr, T **dA_array, const int *ldda_arr,
                 int **ipiv_array, T **dB_array, const int *lddb_arr)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ __align__(16) Diag<T> sD;
     T *sB = reinterpret_cast<T *>(smem);
-    const int k = blockIdx.y, tid = threadIdx.x;
+    const int k = blockIdx.y;
     const int n = n_arr[k], nrhs = nrhs_arr[k];
-    const int c0 = blockIdx.x * VB_NR;
+    const int c0 = blockIdx.x * VB_SOLVE_NR;
     if (n <= 0 || c0 >= nrhs) return;
-    const int nr = min(VB_NR, nrhs - c0);
+    const int nr = min(VB_SOLVE_NR, nrhs - c0), ldx = solve_ldx<T>(n);
+    int *s_piv = reinterpret_cast<int *>(sB + (size_t)VB_SOLVE_NR * ldx);
     const int ldb = lddb_arr[k];
     T *B = dB_array[k] + (size_t)c0 * ldb;
-    for (int e = tid; e < VB_NR * n; e += VB_THREADS) {
-        const int c = e / n, i = e % n;
-        sB[c * n + i] = c < nr ? B[i + (size_t)c * ldb] : T(0);
-    }
-    __syncthreads();
-    solve_smem<T, TRANS, VB_NR>(n, dA_array[k], ldda_arr[k], ipiv_array[k], sB, nr);
-    for (int e = tid; e < nr * n; e += VB_THREADS) {
-        const int c = e / n, i = e % n;
-        B[i + (size_t)c * ldb] = sB[c * n + i];
-    }
+    move_rhs<T, false>(n, TRANS ? nullptr : ipiv_array[k], s_piv, B, ldb, sB, ldx, nr, VB_SOLVE_NR);
+    solve_smem<T, TRANS, solve_cg<T, VB_SOLVE_NR>()>(n, dA_array[k], ldda_arr[k], sB, ldx, nr, sD);
+    move_rhs<T, true>(n, TRANS ? ipiv_array[k] : nullptr, s_piv, B, ldb, sB, ldx, nr, VB_SOLVE_NR);
 }
 
 // argument check + maxima, one small kernel: stats = {err_m, err_n, err_ldda, err_lddb,
@@ -250,7 +241,7 @@ size_t vb_smem_bytes(int max_m, int max_n, int max_nrhs)
     if (max_m > 0 && max_n > 0) need = max(need, panel_regs_smem_bytes<T, 1>());
     need = max(need, (size_t)2 * PANEL_NB * (SWAP_W + 1) * sizeof(T));
     need = max(need, (size_t)(PANEL_NB + GEMM_LDU) * 64 * sizeof(T));
-    if (max_nrhs > 0) need = max(need, (size_t)VB_NR * max_n * sizeof(T));
+    if (max_nrhs > 0) need = max(need, (size_t)VB_NR * solve_ldx<T>(max_n) * sizeof(T));
     return min(need, VB_SMEM_CAP);
 }
 
@@ -329,15 +320,15 @@ magma_int_t vb_getrs_run(bool trans, const int *n, const int *nrhs, int max_n, i
                          magma_queue_t q)
 {
     if (batch <= 0 || max_n <= 0 || max_nrhs <= 0) return 0;
-    const size_t smem = (size_t)VB_NR * max_n * sizeof(T);
-    if (smem > VB_SMEM_CAP) return MAGMA_ERR_NOT_SUPPORTED;
+    if ((size_t)VB_NR * max_n * sizeof(T) > VB_SMEM_CAP) return MAGMA_ERR_NOT_SUPPORTED;
+    const size_t smem = (size_t)VB_SOLVE_NR * solve_ldx<T>(max_n) * sizeof(T) + (size_t)max_n * sizeof(int);
     static size_t dyn_cache[2][MLU_MAX_DEVICES];
     const size_t dyn_max = trans ? mlu_device_cached(dyn_cache[1], [] { return mlu_allow_dynamic_smem(vb_getrs_kernel<T, true>); })
                                  : mlu_device_cached(dyn_cache[0], [] { return mlu_allow_dynamic_smem(vb_getrs_kernel<T, false>); });
     if (smem > dyn_max) return MAGMA_ERR_NOT_SUPPORTED;
     for (int b0 = 0; b0 < batch; b0 += MLU_MAX_GRID_Y) {
         const int nb = min(batch - b0, (int)MLU_MAX_GRID_Y);
-        dim3 grid((max_nrhs + VB_NR - 1) / VB_NR, nb);
+        dim3 grid((max_nrhs + VB_SOLVE_NR - 1) / VB_SOLVE_NR, nb);
         if (trans)
             MLU_LAUNCH(mlu::KC_GETRS, q->stream, vb_getrs_kernel<T, true><<<grid, VB_THREADS, smem, q->stream>>>(
                 n + b0, nrhs + b0, dA + b0, ldda + b0, ipiv + b0, dB + b0, lddb + b0));
