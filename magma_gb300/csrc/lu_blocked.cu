@@ -31,6 +31,7 @@
 #include "trace.cuh"
 #include "lu_core.cuh"
 #include "solve_core.cuh"
+#include "lu_cta.cuh"
 
 #include <type_traits>
 
@@ -558,6 +559,27 @@ static void launch_panel(int rpt, int m, int n, int j0, int ib, T **dA, int ldda
             m, n, j0, ib, dA, ldda, ipiv, info, vs));
 }
 
+// The whole factorisation of a matrix of at most NT rows and columns by one CTA
+// of NT threads (lu_cta.cuh); dynamic shared memory cta_lu_smem.
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, 768 / NT)
+lu_cta_kernel(int m, int n, T **dA_array, int ldda, int **ipiv_array, int *info_array)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(16) CtaPanel<T> s_panel;
+    const int mat = blockIdx.x;
+    cta_lu<T>(m, n, dA_array[mat], ldda, ipiv_array[mat], 0, nullptr, 1, smem_raw, cta_ld(m), cta_ld(n), s_panel, CTA_NB,
+              false, cta_rot(mat), &info_array[mat]);
+}
+
+template <typename T, int NT>
+static void launch_lu_cta(int m, int n, T **dA, int ldda, int **ipiv, int *info, int batch, cudaStream_t s)
+{
+    static size_t dyn_cache[MLU_MAX_DEVICES];
+    mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(lu_cta_kernel<T, NT>); });
+    MLU_LAUNCH(mlu::KC_PANEL, s, lu_cta_kernel<T, NT><<<batch, NT, cta_lu_smem<T>(m, n), s>>>(m, n, dA, ldda, ipiv, info));
+}
+
 static int mlu_sm_count()
 {
     static size_t cache[MLU_MAX_DEVICES];
@@ -763,11 +785,38 @@ static magma_int_t blocked_getrf_outer(int m, int n, T **dA, int ldda, int **ipi
     return MAGMA_SUCCESS;
 }
 
+// Whether the one-CTA kernel (lu_cta.cuh) takes a batch whose larger dimension is
+// n, or the step kernels, which spread a matrix over many CTAs.  Measured per call
+// (step kernels / one CTA, us):
+//   FP64 n=64:  b=8 242 / 222, b=1500 605 / 442;  n=128: b=8 546 / 527, b=1500 3039 / 2198
+//        n=160: b=8 697 / 714, b=76 773 / 718;    n=200: b=8 970 / 1157, b=76 1274 / 1161
+//        n=256: b=76 1753 / 2024, b=152 2407 / 2044, b=1500 18235 / 15777
+//   FP32 n=64:  b=8 163 / 152, b=1500 270 / 208;  n=128: b=8 299 / 271, b=1500 747 / 740
+//        n=200: b=8 480 / 443, b=300 586 / 519, b=600 814 / 1012;  n=256: b=8 574 / 679
+// FP64 is bound by its pipe, which one CTA per SM fills for large orders: above 128
+// the batch has to occupy the SMs.  FP32 above 128 is the other way round: the
+// register-blocked rank-128 updates win once there are two matrices per SM.
+template <typename T>
+static bool one_cta_per_matrix(int n, int batch)
+{
+    if (n > CTA_MAX_N) return false;
+    if (n <= 128) return true;
+    if (sizeof(T) == 8) return (long long)batch * 152 >= (long long)(n - 128) * mlu_sm_count();
+    return n <= 208 && batch <= 2 * mlu_sm_count();
+}
+
 template <typename T>
 magma_int_t blocked_getrf(int m, int n, T **dA, int ldda, int **ipiv, int *info, int batch,
                           magma_queue_t q)
 {
     if (batch <= 0 || m == 0 || n == 0) return MAGMA_SUCCESS;
+    if (ipiv != nullptr && one_cta_per_matrix<T>(max(m, n), batch)) {
+        if (max(m, n) <= 64) launch_lu_cta<T, 64>(m, n, dA, ldda, ipiv, info, batch, q->stream);
+        else if (max(m, n) <= 128) launch_lu_cta<T, 128>(m, n, dA, ldda, ipiv, info, batch, q->stream);
+        else launch_lu_cta<T, 256>(m, n, dA, ldda, ipiv, info, batch, q->stream);
+        MLU_CHECK_LAUNCH();
+        return MAGMA_SUCCESS;
+    }
     if (outer_blocked<T>(m, n))
         return blocked_getrf_outer<T>(m, n, dA, ldda, ipiv, info, batch, q, {nullptr, nullptr, nullptr});
     const int mn = min(m, n);

@@ -11,26 +11,26 @@
 //   1. vb_sort_kernel (one CTA): counting sort of the matrices by size,
 //      largest first, into a work list -- no host round trip;
 //   2. vb_lu_kernel: every CTA repeatedly takes the next matrix of the list
-//      (atomic counter) and runs its complete blocked LU -- panel in shared
-//      memory, interchanges applied to the other columns and to the
-//      right-hand sides, TRSM, 64x64 trailing-update tiles -- then the
+//      (atomic counter) and runs its complete blocked LU (lu_cta.cuh), the
+//      interchanges applied to the right-hand sides on the way, then the
 //      triangular solves.  Largest-first order keeps the SMs evenly loaded to
 //      the end (longest-processing-time scheduling).
-// The steps are the device functions of lu_core.cuh, so factors, pivots and
-// solutions are bit-identical to the fixed-size path and to the CPU oracle.
+// Every step applies the same updates in the same order as the fixed-size path,
+// so factors, pivots and solutions are bit-identical to it and to the CPU oracle.
 // The _max_nocheck_work entry points never allocate or synchronise and can
 // be captured in a CUDA graph.
 #include "common.cuh"
 #include "trace.cuh"
 #include "lu_core.cuh"
 #include "solve_core.cuh"
+#include "lu_cta.cuh"
 
 #include <mutex>
 #include <vector>
 
 namespace mlu {
 
-constexpr int VB_THREADS = PANEL_REGS_THREADS;   // the register panel runs on all threads
+constexpr int VB_THREADS = CTA_MAX_N;      // a thread per row of the panel
 constexpr int VB_BINS = 1024;
 constexpr int VB_NR = 16;                  // right-hand sides per solve pass
 constexpr int VB_SOLVE_NR = 8;             // right-hand sides per CTA of the separate solve
@@ -38,8 +38,10 @@ constexpr size_t VB_SMEM_CAP = 220 * 1024;
 
 // Per-size-bin tuning of the persistent kernel: panel width and trailing-update
 // tile shape for matrices whose max(m, n) falls in bin b (<= 16, 32, 64, 128,
-// 256, 512, 1024, larger).  Every choice applies the same updates to every
-// element in the same order, so the tuning never changes a result.
+// 256, 512, 1024, larger).  Widths above CTA_NB run as CTA_NB; the 32 x 32 tile
+// is 2 x 2 elements per thread in every update, the others 4 x 4.  Every choice
+// applies the same updates to every element in the same order, so the tuning
+// never changes a result.
 constexpr int VB_TUNE_BINS = 8;
 // Batches whose largest matrix is at most this run in the persistent kernel
 // (one CTA per matrix); larger ones in the per-step kernels of the fixed-size
@@ -57,16 +59,6 @@ __host__ __device__ inline int vb_tune_bin(int mx)
     int b = 0;
     for (int ub = 16; b < VB_TUNE_BINS - 1 && mx > ub; ub <<= 1) b++;
     return b;
-}
-
-// all tiles of the trailing update of one step, BM x BN tiles
-template <typename T, int BM, int BN, int TM, int TN>
-__device__ __forceinline__ void vb_update(T *A, int lda, int m, int n, int j0, int ib, T *sL, T *sU)
-{
-    const int rm = m - j0 - ib, rn = n - j0 - ib;
-    for (int tn = 0; tn < rn; tn += BN)
-        for (int tm = 0; tm < rm; tm += BM)
-            gemm_tile<T, BM, BN, TM, TN>(A, lda, m, n, j0, ib, j0 + ib + tm, j0 + ib + tn, sL, sU);
 }
 
 __device__ __forceinline__ int vb_key(int m, int n) { return min(max(max(m, n), 0), VB_BINS - 1); }
@@ -112,18 +104,22 @@ vb_sort_kernel(const int *m_arr, const int *n_arr, int batch, int *order, int *c
     if (tid == 0) *counter = 0;
 }
 
+// Three CTAs per SM (80 registers a thread): the serial steps of one matrix run
+// beside the updates of two others.
 template <typename T>
-__global__ void __launch_bounds__(VB_THREADS, 2)
+__global__ void __launch_bounds__(VB_THREADS, 3)
 vb_lu_kernel(const int *m_arr, const int *n_arr, const int *nrhs_arr, T **dA_array,
              const int *ldda_arr, int **ipiv_array, T **dB_array, const int *lddb_arr,
-             int *info_array, const int *order, int *counter, int batch, int smem_bytes,
+             int *info_array, const int *order, int *counter, int batch, int ldp, int ldu,
              VbTune tune)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ __align__(16) Diag<T> sD;
-    __shared__ int s_item, s_ipiv[PANEL_NB], s_row[2 * PANEL_NB], s_src[2 * PANEL_NB], s_cnt;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    T *sT = reinterpret_cast<T *>(smem);
+    __shared__ __align__(16) CtaPanel<T> s_panel;
+    __shared__ int s_item;
+    const int tid = threadIdx.x;
+    // the solve's diagonal block, then its right-hand sides, in the same memory
+    Diag<T> &sD = *reinterpret_cast<Diag<T> *>(smem);
+    T *sT = reinterpret_cast<T *>(smem + sizeof(Diag<T>));
     for (;;) {
         __syncthreads();
         if (tid == 0) s_item = atomicAdd(counter, 1);
@@ -134,49 +130,11 @@ vb_lu_kernel(const int *m_arr, const int *n_arr, const int *nrhs_arr, T **dA_arr
         const int m = m_arr[k], n = n_arr[k], lda = ldda_arr[k];
         const int nrhs = nrhs_arr ? nrhs_arr[k] : 0;
         T *A = dA_array[k];
-        int *ipiv = ipiv_array[k];
         T *B = nrhs > 0 ? dB_array[k] : nullptr;
         const int ldb = nrhs > 0 ? lddb_arr[k] : 1;
-        const int mn = min(m, n);
         const int bin = vb_tune_bin(max(m, n));
-        const int nbw = tune.nb[bin], tile = tune.tile[bin];
-        int info = 0;
-        for (int j0 = 0; j0 < mn;) {
-            const int pm = m - j0;
-            // register-resident panel (one row per thread) when pm <= 256, else
-            // the shared-memory panel
-            const int ib = pm <= VB_THREADS ? min(nbw, mn - j0)
-                                            : panel_width<T>(pm, min(nbw, mn - j0),
-                                                             (size_t)smem_bytes);
-            T *Ap = A + j0 + (size_t)j0 * lda;
-            const int il = pm <= VB_THREADS ? panel_factor_regs<T, 1>(pm, ib, Ap, lda, s_ipiv, j0,
-                                                                      smem)
-                                            : panel_factor<T>(pm, ib, Ap, lda, smem, s_ipiv, j0);
-            if (info == 0) info = il;
-            if (tid < ib) ipiv[j0 + tid] = j0 + s_ipiv[tid] + 1;
-            __syncthreads();
-            if (warp == 0) build_permutation(ipiv, j0, ib, s_row, s_src, &s_cnt);
-            __syncthreads();
-            const int cnt = s_cnt;
-            if (cnt > 0) {
-                apply_permutation<T>(A, lda, 0, j0, s_row, s_src, cnt, sT);
-                apply_permutation<T>(A, lda, j0 + ib, n, s_row, s_src, cnt, sT);
-                if (nrhs > 0) apply_permutation<T>(B, ldb, 0, nrhs, s_row, s_src, cnt, sT);
-            }
-            if (j0 + ib < n) {
-                trsm_l11_smem<T>(A, lda, j0, ib, j0 + ib, n, sT, 64);
-                T *sL = sT, *sU = sT + PANEL_NB * 64;
-                if (tile == VB_TILE_32x32)
-                    vb_update<T, 32, 32, 2, 2>(A, lda, m, n, j0, ib, sL, sU);
-                else if (tile == VB_TILE_32x64)
-                    vb_update<T, 32, 64, 2, 4>(A, lda, m, n, j0, ib, sL, sU);
-                else
-                    vb_update<T, 64, 64, 4, 4>(A, lda, m, n, j0, ib, sL, sU);
-                __syncthreads();
-            }
-            j0 += ib;
-        }
-        if (tid == 0) info_array[k] = info;
+        cta_lu<T>(m, n, A, lda, ipiv_array[k], nrhs, B, ldb, smem, ldp, ldu, s_panel,
+                  min((int)tune.nb[bin], CTA_NB), tune.tile[bin] == VB_TILE_32x32, cta_rot(idx), &info_array[k]);
         if (nrhs > 0 && m == n && n > 0) {
             const int ldx = solve_ldx<T>(n);
             for (int c0 = 0; c0 < nrhs; c0 += VB_NR) {
@@ -234,15 +192,9 @@ __global__ void vb_check_kernel(const int *m, const int *n, const int *nrhs, con
 template <typename T>
 size_t vb_smem_bytes(int max_m, int max_n, int max_nrhs)
 {
-    size_t need = 0;
-    const int pm = max(max_m, 1);
-    if (pm > VB_THREADS)   // shorter panels live in registers
-        need = max(need, panel_smem_bytes<T>(pm, min(PANEL_NB, max(min(max_m, max_n), 1))));
-    if (max_m > 0 && max_n > 0) need = max(need, panel_regs_smem_bytes<T, 1>());
-    need = max(need, (size_t)2 * PANEL_NB * (SWAP_W + 1) * sizeof(T));
-    need = max(need, (size_t)(PANEL_NB + GEMM_LDU) * 64 * sizeof(T));
-    if (max_nrhs > 0) need = max(need, (size_t)VB_NR * solve_ldx<T>(max_n) * sizeof(T));
-    return min(need, VB_SMEM_CAP);
+    size_t need = cta_lu_smem<T>(max(max_m, 1), max(max_n, 1));
+    if (max_nrhs > 0) need = max(need, sizeof(Diag<T>) + (size_t)VB_NR * solve_ldx<T>(max_n) * sizeof(T));
+    return need;
 }
 
 size_t vb_work_bytes(int batch) { return ((size_t)batch * sizeof(int) + 16 + 255) & ~(size_t)255; }
@@ -287,13 +239,8 @@ magma_int_t vb_run(const int *m, const int *n, const int *nrhs, int max_m, int m
     }
     static size_t dyn_cache[MLU_MAX_DEVICES];
     const size_t dyn_max = mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(vb_lu_kernel<T>); });
-    const size_t smem = min(vb_smem_bytes<T>(max_m, max_n, max_nrhs), dyn_max);
-    // the panel of the largest matrix must fit with at least width 1
-    if (max_m > VB_THREADS && panel_smem_bytes<T>(max_m, 1) > smem)
-        return MAGMA_ERR_NOT_SUPPORTED;
-    if ((size_t)(PANEL_NB + GEMM_LDU) * 64 * sizeof(T) > smem) return MAGMA_ERR_NOT_SUPPORTED;
-    if (max_m > 0 && max_n > 0 && panel_regs_smem_bytes<T, 1>() > smem) return MAGMA_ERR_NOT_SUPPORTED;
-    if (max_nrhs > 0 && (size_t)VB_NR * max_n * sizeof(T) > smem) return MAGMA_ERR_NOT_SUPPORTED;
+    const size_t smem = vb_smem_bytes<T>(max_m, max_n, max_nrhs);   // 68 KB at most
+    if (smem > dyn_max) return MAGMA_ERR_NOT_SUPPORTED;
     int *order = (int *)work;
     int *counter = (int *)((char *)work + vb_work_bytes(batch) - 16);
     MLU_LAUNCH(mlu::KC_OTHER, q->stream, vb_sort_kernel<<<1, 1024, 0, q->stream>>>(m, n, batch, order, counter));
@@ -302,7 +249,7 @@ magma_int_t vb_run(const int *m, const int *n, const int *nrhs, int max_m, int m
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vb_lu_kernel<T>, VB_THREADS, smem);
     const int grid = max(1, min(batch, sms * max(per_sm, 1)));
     MLU_LAUNCH(mlu::KC_VB_LU, q->stream, vb_lu_kernel<T><<<grid, VB_THREADS, smem, q->stream>>>(m, n, nrhs, dA, ldda, ipiv, dB, lddb, info,
-                                                          order, counter, batch, (int)smem, tune));
+                                                          order, counter, batch, cta_ld(max(max_m, 1)), cta_ld(max(max_n, 1)), tune));
     MLU_CHECK_LAUNCH();
     return 0;
 }
