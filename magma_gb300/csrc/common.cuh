@@ -38,15 +38,18 @@ template <> struct Prec<double> {
     __device__ static inline bool normal_or_special(double x) {
         return (__double2hiint(x) & 0x7ff00000) != 0;
     }
+    // On the two 32-bit halves: the same tests on the 64-bit pattern are recognised
+    // as floating-point comparisons and compiled to FP64 instructions (three of them
+    // in a pivot step, as much of the pipe as three FMAs).
     __device__ static inline bool nonzero(double x) {
-        return ((__double_as_longlong(x) << 1) != 0);
+        return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) != 0u;
     }
     __device__ static inline bool isnan_(double x) {
-        return (((unsigned long long)__double_as_longlong(x)) << 1) > (0x7ff0000000000000ull << 1);
+        return (((unsigned)__double2hiint(x) & 0x7fffffffu) | (__double2loint(x) != 0 ? 1u : 0u)) > 0x7ff00000u;
     }
     // |x| as a 63-bit unsigned key (monotone in |x| for non-NaN x).
     __device__ static inline unsigned long long absbits(double x) {
-        return ((unsigned long long)__double_as_longlong(x)) & 0x7fffffffffffffffull;
+        return ((unsigned long long)((unsigned)__double2hiint(x) & 0x7fffffffu) << 32) | (unsigned)__double2loint(x);
     }
     __device__ static inline double fma_(double a, double b, double c) { return fma(a, b, c); }
 };

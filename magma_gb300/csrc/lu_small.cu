@@ -16,49 +16,43 @@
 // current position.  NaN follows idamax's strict '>' scan: a NaN at the
 // current diagonal position wins, any other NaN never does.
 //
-// GB300 note: FP64 issues at a small fraction of the FP32 rate on this part,
-// so the kernel keeps everything except the eliminations themselves (pivot
-// search, interchanges, broadcasts) off the FP64 pipe, and the U solve reuses
-// the pivot reciprocals computed during the factorisation.
+// FP64 keeps the matrix in shared memory instead (small_gesv_packed_kernel): an
+// FP64 warp instruction takes 16 cycles of the SM's FP64 pipe whatever its lanes
+// do, so the trailing elements of a step are spread over all 32 lanes.
 #include "common.cuh"
 #include "trace.cuh"
 
 namespace mlu {
 
-constexpr int SMALL_WARPS = 4;   // matrices per CTA (solve kernel)
-constexpr int GESV_WARPS = 8;    // matrices per CTA (factor kernel, lockstep)
+constexpr int SMALL_WARPS = 4;   // matrices per CTA (solve kernel, packed factor kernel)
+constexpr int GESV_WARPS = 8;    // matrices per CTA (register factor kernel)
 
-// The factor kernel runs its GESV_WARPS warps in lockstep so that the pivot
-// reciprocals of all of them come from one FP64 division sequence issued by
-// warp 0 (one lane per matrix): on this part the FP64 pipe, not latency, is
-// the limit, and a division costs as many FP64 issue slots whether one lane or
-// thirty-two use it.
+// FP32: lane = row in registers.
 template <typename T, int N, int NRHS>
-__global__ void __launch_bounds__(GESV_WARPS * 32, 2)
+__global__ void __launch_bounds__(GESV_WARPS * 32, NRHS > 4 ? 2 : 3)
 small_gesv_kernel(int n, int nrhs, T **dA_array, int ldda, int **ipiv_array, T **dB_array,
                   int lddb, int *info_array, int batch)
 {
-    __shared__ T s_piv[GESV_WARPS], s_rcp[GESV_WARPS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int mat = blockIdx.x * GESV_WARPS + warp;
-    const bool live = mat < batch;   // dead warps still take part in the barriers
+    if (mat >= batch) return;
 
-    T *A = live ? dA_array[mat] : nullptr;
+    T *A = dA_array[mat];
     const bool row_valid = lane < n;
 
     T a[N];
 #pragma unroll
     for (int j = 0; j < N; j++)
-        a[j] = (live && row_valid && j < n) ? A[lane + (size_t)j * ldda] : T(0);
+        a[j] = (row_valid && j < n) ? A[lane + (size_t)j * ldda] : T(0);
 
     constexpr int NB = NRHS > 0 ? NRHS : 1;
     T b[NB];
     T *B = nullptr;
     if (NRHS > 0) {
-        B = live ? dB_array[mat] : nullptr;
+        B = dB_array[mat];
 #pragma unroll
         for (int c = 0; c < NB; c++)
-            b[c] = (live && row_valid && c < nrhs) ? B[lane + (size_t)c * lddb] : T(0);
+            b[c] = (row_valid && c < nrhs) ? B[lane + (size_t)c * lddb] : T(0);
     }
 
     unsigned pos = lane;      // position in LAPACK's current row order
@@ -82,11 +76,7 @@ small_gesv_kernel(int n, int nrhs, T **dA_array, int ldda, int **ipiv_array, T *
         const T piv = shfl(v, plane);
         const bool nz = Prec<T>::nonzero(piv);
         if (!nz && info == 0) info = k + 1;
-        if (lane == 0) s_piv[warp] = piv;
-        __syncthreads();
-        if (warp == 0 && lane < GESV_WARPS) s_rcp[lane] = T(1) / s_piv[lane];
-        __syncthreads();
-        const T r = s_rcp[warp];
+        const T r = recip(piv);
         if (lane == k) my_ipiv = (int)ppos + 1;
         const bool was_k = (pos == (unsigned)k);
         if (lane == plane) { pos = k; active = false; my_rcp = r; }
@@ -131,7 +121,7 @@ small_gesv_kernel(int n, int nrhs, T **dA_array, int ldda, int **ipiv_array, T *
         }
     }
 
-    if (live && row_valid) {
+    if (row_valid) {
 #pragma unroll
         for (int j = 0; j < N; j++)
             if (j < n) A[pos + (size_t)j * ldda] = a[j];
@@ -142,142 +132,179 @@ small_gesv_kernel(int n, int nrhs, T **dA_array, int ldda, int **ipiv_array, T *
                 if (c < nrhs) B[pos + (size_t)c * lddb] = b[c];
         }
     }
-    if (live && lane == 0) info_array[mat] = info;
+    if (lane == 0) info_array[mat] = info;
 }
 
-// Packed variant for 16 < n <= 32: the matrix of each warp sits row-major in
-// shared memory and rows are interchanged physically.  The pivot search and
-// the column scaling are lane = row as above, but the rank-1 update of step k
-// spreads the (n-1-k)^2 trailing elements over all 32 lanes (element e of the
-// step: row k+1+e/w, column k+1+e%w, w = n-1-k), so no FP64 instruction runs
-// with the lanes of finished rows idle: 344 warp FMAs for the update of a
-// 32 x 32 matrix instead of 496.  Every element receives the same operations
-// in the same order as in small_gesv_kernel.
-constexpr int PK_LD = 33;
+// e / d for 0 <= e < 1536 and 1 <= d <= 48: (e * small_magic(d)) >> 20.  The magic
+// number is at least 2^20 / d and less than 2 above it, so that e times its excess
+// stays below 2^20 / d.
+__device__ __forceinline__ unsigned small_magic(int d) { return (unsigned)__fdividef(1048576.f, (float)d) + 1u; }
+__device__ __forceinline__ int small_div(int e, unsigned magic) { return (int)(((unsigned)e * magic) >> 20); }
+
+// FP64, one warp per matrix: the matrix and its right-hand sides sit row-major in
+// shared memory (row stride ld odd, right-hand sides in columns n ..), rows are
+// interchanged physically, and the update of step k spreads its (n-1-k) x
+// (n-1-k+nrhs) elements over all lanes.  Bound by the FP64 pipe: at n = 32 and
+// one right-hand side 356 update FMAs, 31 scalings and 64 solve instructions per
+// matrix (365 would be the bare minimum); the pipe is busy 77 % of the time with
+// the 24 warps that shared memory has room for, the rest is the chain search -
+// reciprocal - scaling of each step.  No barrier: every warp computes its own
+// reciprocals on the integer pipes (10,000 matrices: 420 us with one FP64 division
+// shared by eight warps in lockstep, 326 us now; n = 16: 189 -> 70 us).
+__host__ __device__ constexpr int small_ld(int n, int nrhs) { return (n + nrhs) | 1; }
+// Elements of shared memory per matrix: the rows and the pivot reciprocals (in the
+// padding column where there is one).
+__host__ __device__ constexpr int small_elems(int n, int nrhs)
+{
+    return n * small_ld(n, nrhs) + ((n + nrhs) & 1 ? n : 0);
+}
 
 template <typename T>
-__host__ __device__ constexpr size_t packed_warp_elems(int nb)
-{
-    return (size_t)32 * PK_LD + (size_t)32 * nb + 32;
-}
-
-template <typename T, int NRHS>
-__global__ void __launch_bounds__(GESV_WARPS * 32)
+__global__ void __launch_bounds__(SMALL_WARPS * 32)
 small_gesv_packed_kernel(int n, int nrhs, T **dA_array, int ldda, int **ipiv_array, T **dB_array,
                          int lddb, int *info_array, int batch)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ T s_piv[GESV_WARPS], s_rcp[GESV_WARPS];
-    constexpr int NB = NRHS > 0 ? NRHS : 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int mat = blockIdx.x * GESV_WARPS + warp;
-    const bool live = mat < batch;   // dead warps still take part in the barriers
-    T *sA = reinterpret_cast<T *>(smem_raw) + (size_t)warp * packed_warp_elems<T>(NB);  // [32][PK_LD]
-    T *sB = sA + 32 * PK_LD;                                                           // [32][NB]
-    T *sR = sB + 32 * NB;                                                              // pivot reciprocals
-    const bool row_valid = lane < n;
-    T *A = live ? dA_array[mat] : nullptr;
+    const int mat = blockIdx.x * SMALL_WARPS + warp;
+    if (mat >= batch) return;
+    const int ld = small_ld(n, nrhs), cols = n + nrhs;
+    T *sA = reinterpret_cast<T *>(smem_raw) + (size_t)warp * small_elems(n, nrhs), *sR = (cols & 1) ? sA + n * ld : sA + cols;
+    const int rs = (cols & 1) ? 1 : ld;              // sR[k * rs]: the reciprocal of pivot k
+    T *A = dA_array[mat];
+    T *B = nrhs > 0 ? dB_array[mat] : nullptr;
+    const unsigned mn = small_magic(n);
 #pragma unroll 8
-    for (int j = 0; j < 32; j++)
-        sA[lane * PK_LD + j] = (live && row_valid && j < n) ? A[lane + (size_t)j * ldda] : T(0);
-    // one right-hand side lives in column 32 of sA (the row padding), so that its
-    // update rides in the packed update of each step
-    auto bref = [&](int row, int c) -> T & { return NRHS == 1 ? sA[row * PK_LD + 32] : sB[row * NB + c]; };
-    T *B = nullptr;
-    if (NRHS > 0) {
-        B = live ? dB_array[mat] : nullptr;
-#pragma unroll
-        for (int c = 0; c < NB; c++)
-            bref(lane, c) = (live && row_valid && c < nrhs) ? B[lane + (size_t)c * lddb] : T(0);
+    for (int e = lane; e < n * n; e += 32) {
+        const int j = small_div(e, mn), i = e - j * n;
+        sA[i * ld + j] = A[i + (size_t)j * ldda];
+    }
+#pragma unroll 4
+    for (int e = lane; e < n * nrhs; e += 32) {
+        const int c = small_div(e, mn), i = e - c * n;
+        sA[i * ld + n + c] = B[i + (size_t)c * lddb];
     }
     __syncwarp();
     int info = 0, my_ipiv = 0;
+    bool plain = true;                               // no pivot needs the division
     for (int k = 0; k < n; k++) {
-        const T v = sA[lane * PK_LD + k];
-        const bool cand = lane >= k && row_valid;
+        const bool cand = lane >= k && lane < n;
+        T *vp = sA + min(lane, n - 1) * ld + k;      // this lane's entry of column k
+        const T v = *vp;
         unsigned long long key = 0ull;
         if (cand) {
             unsigned long long mag = Prec<T>::absbits(v);
             if (Prec<T>::isnan_(v)) mag = (lane == k) ? 0x7fffffffffffffffull : 0ull;
             key = mag | 0x8000000000000000ull;
         }
-        const int p = (int)warp_argmax_key(key, cand ? (unsigned)lane : 0xffffffffu);
+        const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+        const unsigned mhi = __reduce_max_sync(FULL, hi);
+        unsigned win = __ballot_sync(FULL, cand && hi == mhi);
+        if (win & (win - 1)) {                       // upper halves tie
+            const unsigned mlo = __reduce_max_sync(FULL, hi == mhi ? lo : 0u);
+            win = __ballot_sync(FULL, cand && hi == mhi && lo == mlo);
+        }
+        const int p = __ffs(win) - 1;                // the smallest position among equals
         const T piv = shfl(v, p);
         const bool nz = Prec<T>::nonzero(piv);
         if (!nz && info == 0) info = k + 1;
-        if (lane == k) my_ipiv = p + 1;
-        if (p != k && MLU_BC2(p, 0, n, 1, 601)) {       // whole rows k and p, and the right-hand sides
-            if (row_valid) {
-                const T x = sA[k * PK_LD + lane];
-                sA[k * PK_LD + lane] = sA[p * PK_LD + lane];
-                sA[p * PK_LD + lane] = x;
-            }
-            if (NRHS > 0 && lane < NB) {
-                const T x = bref(k, lane);
-                bref(k, lane) = bref(p, lane);
-                bref(p, lane) = x;
+        if (p != k && MLU_BC2(p, 0, n, 1, 601)) {    // whole rows k and p
+            for (int c = lane; c < cols; c += 32) {
+                const T x = sA[k * ld + c];
+                sA[k * ld + c] = sA[p * ld + c];
+                sA[p * ld + c] = x;
             }
         }
-        if (lane == 0) s_piv[warp] = piv;
-        __syncthreads();
-        if (warp == 0 && lane < GESV_WARPS) s_rcp[lane] = T(1) / s_piv[lane];
-        __syncthreads();
-        const T r = s_rcp[warp];
-        if (lane == 0) sR[k] = r;
-        if (lane > k && row_valid && nz) sA[lane * PK_LD + k] = rscale(sA[lane * PK_LD + k], piv, r);
+        if (lane == k) my_ipiv = p + 1;
+        plain = plain && Prec<T>::normal_or_special(piv);
+        const T r = recip(piv);
+        if (lane == 0) sR[k * rs] = r;
         __syncwarp();
-        const int w = n - 1 - k;
+        if (cand && lane > k && nz) *vp = rscale(*vp, piv, r);
+        __syncwarp();
+        const int w = n - 1 - k, wc = w + nrhs;
         if (w > 0) {
-            // rows k+1.. by columns k+1..n-1, and column 32 (b) with one right-hand side
-            const int wc = NRHS == 1 ? w + 1 : w;
-            const float inv = 1.0f / (float)wc;
-            for (int e = lane; e < w * wc; e += 32) {
-                int i = __float2int_rz((float)e * inv);
-                int j = e - i * wc;
-                if (j < 0) { i--; j += wc; } else if (j >= wc) { i++; j -= wc; }
-                const int col = (NRHS == 1 && j == w) ? 32 : k + 1 + j;
-                T *dst = sA + (k + 1 + i) * PK_LD + col;
-                *dst = Prec<T>::fma_(-sA[(k + 1 + i) * PK_LD + k], sA[k * PK_LD + col], *dst);
-            }
-            if (NRHS > 1 && lane > k && row_valid) {
+            // element e: row k+1 + e / wc, column k+1 + e % wc
+            const unsigned mw = small_magic(wc);
+            const T *uk = sA + k * ld + k + 1;       // the pivot row right of the pivot
+            T *base = sA + (k + 1) * ld + k;         // row k+1, column k (the multipliers)
+            const int total = w * wc;
+            int e = lane;
+            // four elements at a time, their loads ahead of their stores
+            for (int e0 = 0; e0 + 128 <= total; e0 += 128, e += 128) {
+                T *d[4], l[4], u[4], a[4];
 #pragma unroll
-                for (int c = 0; c < NB; c++)
-                    if (c < nrhs)
-                        sB[lane * NB + c] = Prec<T>::fma_(-sA[lane * PK_LD + k], sB[k * NB + c], sB[lane * NB + c]);
+                for (int q = 0; q < 4; q++) {
+                    const int i = small_div(e + 32 * q, mw), j = e + 32 * q - i * wc;
+                    T *row = base + i * ld;
+                    l[q] = row[0];
+                    u[q] = uk[j];
+                    d[q] = row + 1 + j;
+                    a[q] = *d[q];
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) *d[q] = Prec<T>::fma_(-l[q], u[q], a[q]);
+            }
+            // (not unrolled: guarded copies would be predicated, and an FP64
+            // instruction that is predicated off takes its time in the pipe)
+#pragma unroll 1
+            for (; e < total; e += 32) {
+                const int i = small_div(e, mw), j = e - i * wc;
+                T *row = base + i * ld;
+                row[1 + j] = Prec<T>::fma_(-row[0], uk[j], row[1 + j]);
             }
         }
         __syncwarp();
     }
-    if (NRHS > 0) {
-        // U x = y, lane = row, multiplying by the stored pivot reciprocals
-        for (int t = n - 1; t >= 0; t--) {
-            const T d = sA[t * PK_LD + t], rr = sR[t];
-            T x[NB];
-#pragma unroll
-            for (int c = 0; c < NB; c++) x[c] = rscale(bref(t, c), d, rr);
-            __syncwarp();
-#pragma unroll
-            for (int c = 0; c < NB; c++) {
-                if (c < nrhs) {
-                    if (lane == t) bref(t, c) = x[c];
-                    else if (lane < t) bref(lane, c) = Prec<T>::fma_(-sA[lane * PK_LD + t], x[c], bref(lane, c));
+    if (nrhs > 0) {
+        // U x = y, multiplying by the pivot reciprocals
+        if (nrhs == 1) {                             // lane = row, y in registers
+            const T *row = sA + min(lane, n - 1) * ld;
+            T y = row[n];
+            if (plain) {
+#pragma unroll 4
+                for (int t = n - 1; t >= 0; t--) {
+                    const T x = shfl(y, t) * sR[t * rs], z = Prec<T>::fma_(-row[t], x, y);
+                    y = lane == t ? x : lane < t ? z : y;
+                }
+            } else {
+#pragma unroll 1
+                for (int t = n - 1; t >= 0; t--) {
+                    const T x = rscale(shfl(y, t), sA[t * ld + t], sR[t * rs]), z = Prec<T>::fma_(-row[t], x, y);
+                    y = lane == t ? x : lane < t ? z : y;
                 }
             }
-            __syncwarp();
+            if (lane < n) sA[lane * ld + n] = y;
+        } else {
+            const unsigned mr = small_magic(nrhs);
+            for (int t = n - 1; t >= 0; t--) {
+                const T r = sR[t * rs], d = sA[t * ld + t];
+                T *xt = sA + t * ld + n;
+                if (lane < nrhs) xt[lane] = plain ? xt[lane] * r : rscale(xt[lane], d, r);
+                __syncwarp();
+#pragma unroll 1
+                for (int e = lane; e < t * nrhs; e += 32) {
+                    const int i = small_div(e, mr), c = e - i * nrhs;
+                    T *y = sA + i * ld + n + c;
+                    *y = Prec<T>::fma_(-sA[i * ld + t], xt[c], *y);
+                }
+                __syncwarp();
+            }
         }
+        __syncwarp();
     }
-    if (live && row_valid) {
 #pragma unroll 8
-        for (int j = 0; j < 32; j++)
-            if (j < n) A[lane + (size_t)j * ldda] = sA[lane * PK_LD + j];
-        ipiv_array[mat][lane] = my_ipiv;
-        if (NRHS > 0) {
-#pragma unroll
-            for (int c = 0; c < NB; c++)
-                if (c < nrhs) B[lane + (size_t)c * lddb] = bref(lane, c);
-        }
+    for (int e = lane; e < n * n; e += 32) {
+        const int j = small_div(e, mn), i = e - j * n;
+        A[i + (size_t)j * ldda] = sA[i * ld + j];
     }
-    if (live && lane == 0) info_array[mat] = info;
+#pragma unroll 4
+    for (int e = lane; e < n * nrhs; e += 32) {
+        const int c = small_div(e, mn), i = e - c * n;
+        B[i + (size_t)c * lddb] = sA[i * ld + n + c];
+    }
+    if (lane < n) ipiv_array[mat][lane] = my_ipiv;
+    if (lane == 0) info_array[mat] = info;
 }
 
 // Solve with existing factors, n <= 32.  NoTrans: lane i holds row i of LU.
@@ -395,18 +422,6 @@ template <typename T, int N, int NRHS>
 static void launch_small_gesv(int n, int nrhs, T **dA, int ldda, int **ipiv, T **dB, int lddb,
                               int *info, int batch, cudaStream_t s)
 {
-    if (N == 32) {   // 16 < n <= 32: the packed shared-memory kernel
-        constexpr int NB = NRHS > 0 ? NRHS : 1;
-        const size_t smem = (size_t)GESV_WARPS * packed_warp_elems<T>(NB) * sizeof(T);
-        static size_t dyn_cache[MLU_MAX_DEVICES];
-        const size_t dyn = mlu_device_cached(
-            dyn_cache, [] { return mlu_allow_dynamic_smem(small_gesv_packed_kernel<T, NRHS>); });
-        if (smem <= dyn) {
-            MLU_LAUNCH(mlu::KC_SMALL_GESV, s, small_gesv_packed_kernel<T, NRHS><<<mlu_ceildiv(batch, GESV_WARPS), GESV_WARPS * 32, smem, s>>>(
-                n, nrhs, dA, ldda, ipiv, dB, lddb, info, batch));
-            return;
-        }
-    }
     MLU_LAUNCH(mlu::KC_SMALL_GESV, s, small_gesv_kernel<T, N, NRHS><<<mlu_ceildiv(batch, GESV_WARPS), GESV_WARPS * 32, 0, s>>>(
         n, nrhs, dA, ldda, ipiv, dB, lddb, info, batch));
 }
@@ -429,9 +444,17 @@ magma_int_t small_gesv(int n, int nrhs, T **dA, int ldda, int **ipiv, T **dB, in
     if (n > 32 || n < 1 || nrhs > 16) return MAGMA_ERR;   // -100: not applicable
     if (batch <= 0) return MAGMA_SUCCESS;
     cudaStream_t s = q->stream;
-    if (n <= 8)       dispatch_nrhs<T, 8>(n, nrhs, dA, ldda, ipiv, dB, lddb, info, batch, s);
-    else if (n <= 16) dispatch_nrhs<T, 16>(n, nrhs, dA, ldda, ipiv, dB, lddb, info, batch, s);
-    else              dispatch_nrhs<T, 32>(n, nrhs, dA, ldda, ipiv, dB, lddb, info, batch, s);
+    if constexpr (sizeof(T) == 8) {
+        const size_t smem = (size_t)SMALL_WARPS * small_elems(n, nrhs) * sizeof(T);   // at most 52 KB
+        static size_t dyn_cache[MLU_MAX_DEVICES];
+        mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(small_gesv_packed_kernel<T>); });
+        MLU_LAUNCH(mlu::KC_SMALL_GESV, s, small_gesv_packed_kernel<T><<<mlu_ceildiv(batch, SMALL_WARPS), SMALL_WARPS * 32, smem, s>>>(
+            n, nrhs, dA, ldda, ipiv, dB, lddb, info, batch));
+    } else {
+        if (n <= 8)       dispatch_nrhs<T, 8>(n, nrhs, dA, ldda, ipiv, dB, lddb, info, batch, s);
+        else if (n <= 16) dispatch_nrhs<T, 16>(n, nrhs, dA, ldda, ipiv, dB, lddb, info, batch, s);
+        else              dispatch_nrhs<T, 32>(n, nrhs, dA, ldda, ipiv, dB, lddb, info, batch, s);
+    }
     MLU_CHECK_LAUNCH();
     return MAGMA_SUCCESS;
 }
