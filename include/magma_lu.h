@@ -148,6 +148,13 @@ void magma_sset_pointer(float **output_array, float *input, magma_int_t lda,
 void magma_iset_pointer(magma_int_t **output_array, magma_int_t *input, magma_int_t lda,
                         magma_int_t row, magma_int_t column, magma_int_t batch_offset,
                         magma_int_t batchCount, magma_queue_t queue);
+/* No counterpart in the reference: up to six such arrays in one launch.  Entry k
+ * of array a, at output_arrays[a * batchCount + k] (device memory), is bases[a] +
+ * k * strides[a] bytes.  Returns -2 for more than six arrays, -5 for a negative
+ * batch. */
+magma_int_t magma_lu_set_pointers(void **output_arrays, magma_int_t arrays, const void *const *bases,
+                                  const size_t *strides, magma_int_t batchCount, magma_queue_t queue);
+
 
 /* ------------------------------------------------------------------------ */
 /* Batched LU, fixed size -- include/magma_zbatched.h                       */

@@ -9,12 +9,10 @@ No refactorisation happens in the backward pass.  FP64 and FP32 CUDA tensors.
 """
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
 from . import lib as _L
-from .batched import Queue, _check, _prefix, _vp, gesv_batched, ptr_array
+from .batched import Queue, _check, _prefix, _ptrs, gesv_batched
 
 
 class BatchedSolve(torch.autograd.Function):
@@ -40,10 +38,9 @@ class BatchedSolve(torch.autograd.Function):
         GA = torch.empty((b, n, n), dtype=S.dtype, device=S.device)   # storage of gA
         lib = _L.load()
         q = Queue.current(S.device)
-        dS, dP, dX, dG, dGA = ptr_array(S), ptr_array(ipiv), ptr_array(X), ptr_array(G), \
-            ptr_array(GA)
+        dS, dP, dX, dG, dGA, _keep = _ptrs(q, S, ipiv, X, G, GA)
         rc = getattr(lib, f"magma_{_prefix(S)}gesv_adjoint_batched")(
-            n, nrhs, _vp(dS), n, _vp(dP), _vp(dX), n, _vp(dG), n, _vp(dGA), n, b, q.handle)
+            n, nrhs, dS, n, dP, dX, n, dG, n, dGA, n, b, q.handle)
         _check(rc, "magma_gesv_adjoint_batched")
         gA = GA.transpose(1, 2) if ctx.needs_input_grad[0] else None
         gB = G.transpose(1, 2) if ctx.needs_input_grad[1] else None

@@ -83,6 +83,24 @@ def ptr_array(S: torch.Tensor) -> torch.Tensor:
     return S.data_ptr() + torch.arange(S.shape[0], device=S.device, dtype=torch.int64) * step
 
 
+def _ptrs(queue: Queue, *tensors: torch.Tensor) -> list:
+    """The pointer arrays of up to six batches for one call on `queue`, made by one
+    launch: a list of C pointers, and last the tensor that holds them, which must stay
+    referenced until the call has enqueued its kernels."""
+    b, dev = tensors[0].shape[0], tensors[0].device
+    k = len(tensors)
+    if b == 0 or queue.stream_handle != torch.cuda.current_stream(dev).cuda_stream:
+        # another stream than torch's: filled, as before, in the order of torch's own
+        arrays = [ptr_array(t) for t in tensors]
+        return [_vp(a) for a in arrays] + [arrays]
+    out = torch.empty((k, b), dtype=torch.int64, device=dev)
+    bases = (C.c_void_p * k)(*[t.data_ptr() for t in tensors])
+    strides = (C.c_size_t * k)(*[t.stride(0) * t.element_size() for t in tensors])
+    p = out.data_ptr()
+    _check(_L.load().magma_lu_set_pointers(p, k, bases, strides, b, queue.handle), "magma_lu_set_pointers")
+    return [C.c_void_p(p + 8 * b * a) for a in range(k)] + [out]
+
+
 def _prefix(t: torch.Tensor) -> str:
     if t.dtype == torch.float64:
         return "d"
@@ -119,10 +137,8 @@ def getrf_batched(S: torch.Tensor, m: int | None = None, ipiv: torch.Tensor | No
     q = queue or Queue.current(S.device)
     lib = _L.load()
     p = _prefix(S)
-    # the pointer arrays must stay referenced until the call has enqueued its kernels
-    dA = ptr_array(S)
-    dP = ptr_array(ipiv)
-    rc = getattr(lib, f"magma_{p}getrf_batched")(m, n, _vp(dA), ld, _vp(dP), _vp(info), b, q.handle)
+    dA, dP, _keep = _ptrs(q, S, ipiv)
+    rc = getattr(lib, f"magma_{p}getrf_batched")(m, n, dA, ld, dP, _vp(info), b, q.handle)
     _check(rc, f"magma_{p}getrf_batched")
     return ipiv, info
 
@@ -138,9 +154,8 @@ def getrs_batched(LU: torch.Tensor, ipiv: torch.Tensor, B: torch.Tensor, trans: 
     lib = _L.load()
     p = _prefix(LU)
     tr = _L.MagmaTrans if trans else _L.MagmaNoTrans
-    dA, dP, dB = ptr_array(LU), ptr_array(ipiv), ptr_array(B)
-    rc = getattr(lib, f"magma_{p}getrs_batched")(tr, n, nrhs, _vp(dA), ld, _vp(dP), _vp(dB), ldb,
-                                                 b, q.handle)
+    dA, dP, dB, _keep = _ptrs(q, LU, ipiv, B)
+    rc = getattr(lib, f"magma_{p}getrs_batched")(tr, n, nrhs, dA, ld, dP, dB, ldb, b, q.handle)
     _check(rc, f"magma_{p}getrs_batched")
     return B
 
@@ -157,9 +172,8 @@ def gesv_batched(S: torch.Tensor, B: torch.Tensor, ipiv: torch.Tensor | None = N
     q = queue or Queue.current(S.device)
     lib = _L.load()
     p = _prefix(S)
-    dA, dP, dB = ptr_array(S), ptr_array(ipiv), ptr_array(B)
-    rc = getattr(lib, f"magma_{p}gesv_batched")(n, nrhs, _vp(dA), ld, _vp(dP), _vp(dB), ldb,
-                                                _vp(info), b, q.handle)
+    dA, dP, dB, _keep = _ptrs(q, S, ipiv, B)
+    rc = getattr(lib, f"magma_{p}gesv_batched")(n, nrhs, dA, ld, dP, dB, ldb, _vp(info), b, q.handle)
     _check(rc, f"magma_{p}gesv_batched")
     return ipiv, info
 
@@ -199,9 +213,9 @@ def dsgesv_batched(S: torch.Tensor, B: torch.Tensor, X: torch.Tensor | None = No
     if work is None or work.numel() < need:
         work = torch.empty((max(need, 1),), dtype=torch.uint8, device=S.device)
     lw = C.c_size_t(work.numel())
-    dA, dP, dB, dX = ptr_array(S), ptr_array(ipiv), ptr_array(B), ptr_array(X)
-    rc = lib.magma_dxgesv_gmres_batched_work(prec, SOLVERS[solver], n, nrhs, _vp(dA), ld, _vp(dP),
-                                             _vp(dB), ldb, _vp(dX), X.shape[2], _vp(info),
+    dA, dP, dB, dX, _keep = _ptrs(q, S, ipiv, B, X)
+    rc = lib.magma_dxgesv_gmres_batched_work(prec, SOLVERS[solver], n, nrhs, dA, ld, dP,
+                                             dB, ldb, dX, X.shape[2], _vp(info),
                                              _vp(iters), itermax, float(tol), 1 if fallback else 0,
                                              _vp(work), C.byref(lw), b, q.handle)
     _check(rc, "magma_dxgesv_gmres_batched_work")
@@ -233,8 +247,8 @@ def dsposv_batched(S: torch.Tensor, B: torch.Tensor, X: torch.Tensor | None = No
     _check(rc, "magma_dsposv_batched_work(query)")
     work = torch.empty((max(int(lw.value), 1),), dtype=torch.uint8, device=S.device)
     lw = C.c_size_t(work.numel())
-    dA, dB, dX = ptr_array(S), ptr_array(B), ptr_array(X)
-    rc = lib.magma_dsposv_batched_work(122, n, nrhs, _vp(dA), ld, _vp(dB), ldb, _vp(dX),
+    dA, dB, dX, _keep = _ptrs(q, S, B, X)
+    rc = lib.magma_dsposv_batched_work(122, n, nrhs, dA, ld, dB, ldb, dX,
                                        X.shape[2], _vp(info), _vp(iters), itermax, float(tol),
                                        1 if fallback else 0, _vp(work), C.byref(lw), b, q.handle)
     _check(rc, "magma_dsposv_batched_work")
@@ -372,11 +386,14 @@ def dsgesv_adjoint_batched(S: torch.Tensor, ipiv: torch.Tensor, X: torch.Tensor,
     GA = torch.empty((b, n, n), dtype=torch.float64, device=S.device) if want_ga else None
     iters = torch.empty((b,), dtype=torch.int32, device=S.device)
     q = queue or Queue.current(S.device)
-    dA, dP, dX, dG, dGB = ptr_array(S), ptr_array(ipiv), ptr_array(X), ptr_array(G), ptr_array(GB)
-    dGA = ptr_array(GA) if want_ga else None
+    if want_ga:
+        dA, dP, dX, dG, dGB, dGA, _keep = _ptrs(q, S, ipiv, X, G, GB, GA)
+    else:
+        dA, dP, dX, dG, dGB, _keep = _ptrs(q, S, ipiv, X, G, GB)
+        dGA = None
     rc = _L.load().magma_dxgesv_adjoint_batched_work(
-        n, nrhs, _vp(dA), ld, _vp(dP), _vp(dX), X.shape[2], _vp(dG), G.shape[2], _vp(dGB),
-        GB.shape[2], _vp(dGA) if want_ga else None, n, _vp(iters_fwd), _vp(info), _vp(iters),
+        n, nrhs, dA, ld, dP, dX, X.shape[2], dG, G.shape[2], dGB,
+        GB.shape[2], dGA, n, _vp(iters_fwd), _vp(info), _vp(iters),
         itermax, float(tol), int(fallback), _vp(work), work.numel(), b, q.handle)
     _check(rc, "magma_dxgesv_adjoint_batched_work")
     return GB, GA, iters

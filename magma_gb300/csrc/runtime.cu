@@ -185,6 +185,31 @@ extern "C" void magma_iset_pointer(magma_int_t **output_array, magma_int_t *inpu
     set_pointer(output_array, input, lda, row, column, batch_offset, batchCount, queue);
 }
 
+// Up to six arrays of batch pointers, array a at out + a * batch: base[a] + k * stride[a].
+struct PointerBases {
+    unsigned long long base[6], stride[6];
+};
+__global__ void set_pointers_kernel(unsigned long long *out, PointerBases b, int batch) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, a = blockIdx.y;
+    if (k < batch) out[(size_t)a * batch + k] = b.base[a] + (unsigned long long)k * b.stride[a];
+}
+
+extern "C" magma_int_t magma_lu_set_pointers(void **output_arrays, magma_int_t arrays, const void *const *bases,
+                                             const size_t *strides, magma_int_t batchCount, magma_queue_t queue) {
+    if (arrays < 0 || arrays > 6) return -2;
+    if (batchCount < 0) return -5;
+    if (arrays == 0 || batchCount == 0) return 0;
+    PointerBases b = {};
+    for (int a = 0; a < arrays; a++) {
+        b.base[a] = (unsigned long long)bases[a];
+        b.stride[a] = strides[a];
+    }
+    MLU_LAUNCH(mlu::KC_OTHER, queue->stream, set_pointers_kernel<<<dim3(mlu_ceildiv(batchCount, 256), arrays), 256, 0, queue->stream>>>(
+        (unsigned long long *)output_arrays, b, batchCount));
+    MLU_CHECK_LAUNCH();
+    return 0;
+}
+
 #ifdef MLU_BOUNDS_CHECK
 // The bounds-check build's record: the first violation (site << 48 | row << 24
 // | column, each clipped to 24 bits) and the number of violations.

@@ -43,6 +43,7 @@ _PROTOS = {
     "magma_sset_pointer": ([c_ptr, c_ptr, c_int, c_int, c_int, c_int, c_int, c_ptr], None),
     "magma_iset_pointer": ([c_ptr, c_ptr, c_int, c_int, c_int, c_int, c_int, c_ptr], None),
 }
+_PROTOS["magma_lu_set_pointers"] = ([c_ptr, c_int, c_ptr, c_ptr, c_int, c_ptr], c_int)
 for _p in "ds":
     _PROTOS[f"magma_{_p}getrf_batched"] = ([c_int, c_int, c_ptr, c_int, c_ptr, c_ptr, c_int, c_ptr], c_int)
     _PROTOS[f"magma_{_p}getrf_batched_smallsq_noshfl"] = ([c_int, c_ptr, c_int, c_ptr, c_ptr, c_int, c_ptr], c_int)
@@ -158,6 +159,8 @@ KERNEL_CLASSES = {"small_gesv": 1, "panel": 2, "swap_trsm": 3, "gemm": 4, "tc_up
 def load(path: str | os.PathLike | None = None) -> C.CDLL:
     """Load libmagma_lu.so (building it first if the CUDA toolkit is present)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
