@@ -17,14 +17,14 @@
 //                     band right of the panel): the panel's interchanges, the
 //                     solve L11 U12 = A12 and A22 -= L21 U12 for every row
 //                     tile of the band, U12 kept in shared memory;
-//   swap_trsm_kernel  otherwise, one CTA per (matrix, 64-column tile):
+//   right_cols_kernel otherwise, one thread per column right of the panel:
 //     + gemm_kernel   interchanges and U12, then one CTA per 64x64 tile of
 //                     A22 for the update.
 // Every element is updated with one accumulator in increasing k, so the
 // result is bit-identical to the unblocked elimination order.  The
 // interchanges left of each panel are applied after the last step by
 // left_swaps_kernel (one coalesced gather per earlier panel) when the matrix
-// has at most 1024 rows, else by swap_trsm_kernel in each step.
+// has at most 1024 rows, else by left_tile_kernel in each step.
 // No workspace and no host synchronisation: every call is stream-ordered and
 // capturable in a CUDA graph.
 #include "common.cuh"
@@ -67,7 +67,7 @@ panel_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ipiv_ar
 // NT: threads of the CTA (64 or 128 for panels of at most that many rows: fewer
 // warps to synchronise per column, more CTAs per SM).
 template <typename T, int RPT, bool NOPIV = false, int NT = PANEL_THREADS>
-__global__ void __launch_bounds__(NT, (sizeof(T) * RPT * PANEL_NB / 4 > 64) ? 1 : 2)
+__global__ void __launch_bounds__(NT, (NT == 512 || sizeof(T) * RPT * PANEL_NB / 4 > 64) ? 1 : 2)
 panel_regs_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ipiv_array,
                   int *info_array, StepSizes vs)
 {
@@ -98,45 +98,94 @@ __host__ __device__ inline int panel_rows_per_thread(int pm)
     return 0;
 }
 
-// Applies the interchanges of panel [j0, j0+ib) to a SWAP_COLS-column tile
-// outside the panel and, for tiles right of the panel, computes
-// U12 = L11^{-1} A12 (one thread per column).
+// Applies the interchanges of panel [j0, j0+ib) to a SWAP_COLS-column tile left
+// of the panel (matrices too tall for the deferred form, left_swaps_kernel).
 constexpr int SWAP_COLS = 64;
 
 template <typename T>
 __global__ void __launch_bounds__(SWAP_THREADS)
-swap_trsm_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ipiv_array,
-                 StepSizes vs, int with_left, int bj)
+left_tile_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ipiv_array, StepSizes vs)
 {
     __shared__ int s_row[2 * PANEL_NB], s_src[2 * PANEL_NB], s_cnt;
     __shared__ T s_tmp[2 * PANEL_NB * (SWAP_W + 1)];
-    __shared__ T s_rhs[PANEL_NB * SWAP_COLS];
     const int mat = blockIdx.y;
     if (!vs.get(mat, j0, m, n, ldda, ib)) return;
+    const int c0 = blockIdx.x * SWAP_COLS;
+    if (threadIdx.x < 32) build_permutation(ipiv_array[mat], j0, ib, s_row, s_src, &s_cnt);
+    __syncthreads();
+    apply_permutation<T>(dA_array[mat], ldda, c0, min(c0 + SWAP_COLS, j0), s_row, s_src, s_cnt, s_tmp);
+}
+
+// Right of the panel: the interchanges of panel [j0, j0+ib) and U12 = L11^{-1}
+// A12, one thread per column, the column's top block in registers, no barrier
+// after the set-up.  The interchanges as a gather, resolved by each lane running
+// the transpositions backwards: a top row's new content comes from row s_src[k];
+// a row below the top block that an interchange touches ends up holding the
+// original top row s_dsrc[k].  FP64 is bound by the solve's 496 FMAs per column
+// (one FP64 warp instruction per 64 cycles and scheduler), FP32 by the latency of
+// the loads.  n = 512 FP64, 512 matrices: the form with one tile of columns in shared
+// memory (two of four warps solving) took 4260 us per factorisation, this one
+// RIGHT_US; n = 1000 FP32, six matrices: 36 us a step, now RIGHT32_US.
+constexpr int RIGHT_COLS = 64;
+
+template <typename T>
+__global__ void __launch_bounds__(RIGHT_COLS)
+right_cols_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ipiv_array, StepSizes vs, int bj)
+{
+    __shared__ __align__(16) T s_L[PANEL_NB][PANEL_NB];        // [t][i] = L11(i, t)
+    __shared__ int s_src[PANEL_NB], s_dst[PANEL_NB], s_dsrc[PANEL_NB];
+    const int mat = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+    if (!vs.get(mat, j0, m, n, ldda, ib)) return;
     n = block_col_end(bj, m, n);                     // right columns end with the block
+    const int c = j0 + ib + blockIdx.x * RIGHT_COLS + tid;
+    if (j0 + ib + (int)blockIdx.x * RIGHT_COLS >= n) return;   // past this matrix's columns
     T *A = dA_array[mat];
-    // column tile: left tiles cover [0, j0), right tiles cover [j0+ib, n)
-    const int nleft = with_left ? (j0 + SWAP_COLS - 1) / SWAP_COLS : 0;
-    int c0, c1;
-    bool right;
-    if ((int)blockIdx.x < nleft) {
-        c0 = blockIdx.x * SWAP_COLS;
-        c1 = min(c0 + SWAP_COLS, j0);
-        right = false;
-    } else {
-        c0 = j0 + ib + (blockIdx.x - nleft) * SWAP_COLS;
-        c1 = min(c0 + SWAP_COLS, n);
-        right = true;
-        if (c0 >= n) return;             // past this matrix's columns
+    for (int e = tid; e < PANEL_NB * PANEL_NB; e += RIGHT_COLS) {
+        const int i = e % PANEL_NB, t = e / PANEL_NB;
+        s_L[t][i] = i < ib && t < ib ? A[j0 + i + (size_t)(j0 + t) * ldda] : T(0);
     }
-    if (ipiv_array == nullptr) {             // no pivoting: no interchanges
-        if (threadIdx.x == 0) s_cnt = 0;
-    } else if (threadIdx.x < 32) {
-        build_permutation(ipiv_array[mat], j0, ib, s_row, s_src, &s_cnt);
+    if (tid < 32) {
+        int p = j0 + lane;
+        if (ipiv_array != nullptr && lane < ib) p = ipiv_array[mat][j0 + lane] - 1;
+        int vt = j0 + lane, vp = p;
+        for (int k = ib - 1; k >= 0; k--) {
+            const int a = j0 + k, pk = __shfl_sync(FULL, p, k);
+            vt = vt == a ? pk : (vt == pk ? a : vt);
+            vp = vp == a ? pk : (vp == pk ? a : vp);
+        }
+        s_src[lane] = vt;
+        s_dst[lane] = lane < ib && p >= j0 + ib ? p : -1;
+        s_dsrc[lane] = vp;
     }
     __syncthreads();
-    apply_permutation<T>(A, ldda, c0, c1, s_row, s_src, s_cnt, s_tmp);
-    if (right) trsm_l11_smem<T>(A, ldda, j0, ib, c0, c1, s_rhs, SWAP_COLS);
+    if (c >= n) return;
+    T *col = A + (size_t)c * ldda;
+    T v[PANEL_NB];
+#pragma unroll
+    for (int i = 0; i < PANEL_NB; i++)
+        if (i < ib) v[i] = MLU_BC2(s_src[i], c, m, n, 211) ? col[s_src[i]] : T(0);
+    if (ipiv_array != nullptr) {
+#pragma unroll
+        for (int q = 0; q < PANEL_NB; q += 8) {
+            T w[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (s_dst[q + u] >= 0) w[u] = col[s_dsrc[q + u]];
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (s_dst[q + u] >= 0 && MLU_BC2(s_dst[q + u], c, m, n, 212)) col[s_dst[q + u]] = w[u];
+        }
+    }
+    // (a panel narrower than 32 has zero coefficients past its width)
+#pragma unroll
+    for (int t = 0; t < PANEL_NB; t++) {
+        if (t >= ib) break;
+#pragma unroll
+        for (int i = t + 1; i < PANEL_NB; i++) v[i] = Prec<T>::fma_(-s_L[t][i], v[t], v[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < PANEL_NB; i++)
+        if (i < ib) col[j0 + i] = v[i];
 }
 
 // A22 -= L21 * U12 on BM x BN tiles, TM x TN accumulators per thread.
@@ -176,9 +225,9 @@ gemm_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int tiles_m, S
 //      (always a top row: each interchange k moves row j0+k, which still holds
 //      an original top row, down) takes its value from shared memory, so the
 //      interchanges need no scattered writes.
-// Per element the same operations, in the same order, as swap_trsm_kernel
+// Per element the same operations, in the same order, as right_cols_kernel
 // followed by gemm_kernel.  Columns left of the panel are not touched (their
-// interchanges are applied by swap_trsm_kernel or, after the last step, by
+// interchanges are applied by left_tile_kernel or, after the last step, by
 // left_swaps_kernel).
 template <typename T>
 __host__ __device__ int blocked_panel_width(int m, int n, int j0);
@@ -532,6 +581,21 @@ __host__ __device__ int blocked_panel_width(int m, int n, int j0)
     return panel_width<T>(m - j0, want, PANEL_SMEM_MAX);
 }
 
+static int mlu_sm_count()
+{
+    static size_t cache[MLU_MAX_DEVICES];
+    return (int)mlu_device_cached(cache, [] {
+        int dev = 0, count = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            count <= 0) {
+            cudaGetLastError();
+            count = 1;
+        }
+        return (size_t)count;
+    });
+}
+
 // The panel kernel for panels of rpt rows per thread (0: shared memory).
 template <typename T, bool NOPIV>
 static void launch_panel(int rpt, int m, int n, int j0, int ib, T **dA, int ldda, int **ipiv,
@@ -547,12 +611,17 @@ static void launch_panel(int rpt, int m, int n, int j0, int ib, T **dA, int ldda
     else if (rpt == 1)
         MLU_LAUNCH(mlu::KC_PANEL, s, panel_regs_kernel<T, 1, NOPIV><<<nb, PANEL_THREADS, smem, s>>>(
             m, n, j0, ib, dA, ldda, ipiv, info, vs));
-    else if (rpt == 2)
+    else if (rpt == 2 && sizeof(T) == 4 && nb > mlu_sm_count())
+        // two CTAs of two rows per thread on an SM (refinement of 512 matrices of order
+        // 512: 516 us of panels, 778 us with one CTA of a row per thread)
         MLU_LAUNCH(mlu::KC_PANEL, s, panel_regs_kernel<T, 2, NOPIV><<<nb, PANEL_THREADS, smem, s>>>(
+            m, n, j0, ib, dA, ldda, ipiv, info, vs));
+    else if (rpt == 2)
+        MLU_LAUNCH(mlu::KC_PANEL, s, panel_regs_kernel<T, 1, NOPIV, 512><<<nb, 512, smem, s>>>(
             m, n, j0, ib, dA, ldda, ipiv, info, vs));
     else if (rpt == 4)
         MLU_LAUNCH(mlu::KC_PANEL, s,
-                   panel_regs_kernel<T, (sizeof(T) == 4 ? 4 : 2), NOPIV><<<nb, PANEL_THREADS, smem, s>>>(
+                   panel_regs_kernel<T, (sizeof(T) == 4 ? 2 : 1), NOPIV, 512><<<nb, 512, smem, s>>>(
                        m, n, j0, ib, dA, ldda, ipiv, info, vs));
     else
         MLU_LAUNCH(mlu::KC_PANEL, s, panel_kernel<T, NOPIV><<<nb, PANEL_THREADS, smem, s>>>(
@@ -580,25 +649,11 @@ static void launch_lu_cta(int m, int n, T **dA, int ldda, int **ipiv, int *info,
     MLU_LAUNCH(mlu::KC_PANEL, s, lu_cta_kernel<T, NT><<<batch, NT, cta_lu_smem<T>(m, n), s>>>(m, n, dA, ldda, ipiv, info));
 }
 
-static int mlu_sm_count()
-{
-    static size_t cache[MLU_MAX_DEVICES];
-    return (int)mlu_device_cached(cache, [] {
-        int dev = 0, count = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            count <= 0) {
-            cudaGetLastError();
-            count = 1;
-        }
-        return (size_t)count;
-    });
-}
 
 // One step of the blocked factorisation for every matrix: panel at column j0
 // of width ib, interchanges + TRSM, and (when `update`) the trailing update.
 // Right of the panel, band_kernel does all three in one launch (FP32, when the
-// batch gives it at least two CTAs per SM); otherwise swap_trsm_kernel and
+// batch gives it at least two CTAs per SM); otherwise right_cols_kernel and
 // gemm_kernel (more, smaller CTAs) do.  `defer_left`: the interchanges left of
 // the panel are left to left_swaps_kernel after the last step.
 // `vsz`: per-matrix sizes of a variable-size batch (m, n = their maxima).
@@ -617,11 +672,13 @@ magma_int_t blocked_getrf_steps_l(int m, int n, T **dA, int ldda, int **ipiv, in
         const size_t v = min(mlu_allow_dynamic_smem(panel_kernel<T, false>),
                              mlu_allow_dynamic_smem(panel_kernel<T, true>));
         mlu_allow_dynamic_smem(panel_regs_kernel<T, 1, false>);
+        mlu_allow_dynamic_smem(panel_regs_kernel<T, 1, false, 512>);
+        mlu_allow_dynamic_smem(panel_regs_kernel<T, (sizeof(T) == 4 ? 2 : 1), false, 512>);
         mlu_allow_dynamic_smem(panel_regs_kernel<T, 2, false>);
-        mlu_allow_dynamic_smem(panel_regs_kernel<T, (sizeof(T) == 4 ? 4 : 2), false>);
-        mlu_allow_dynamic_smem(panel_regs_kernel<T, 1, true>);
         mlu_allow_dynamic_smem(panel_regs_kernel<T, 2, true>);
-        mlu_allow_dynamic_smem(panel_regs_kernel<T, (sizeof(T) == 4 ? 4 : 2), true>);
+        mlu_allow_dynamic_smem(panel_regs_kernel<T, 1, true>);
+        mlu_allow_dynamic_smem(panel_regs_kernel<T, 1, true, 512>);
+        mlu_allow_dynamic_smem(panel_regs_kernel<T, (sizeof(T) == 4 ? 2 : 1), true, 512>);
         if (band_used<T>()) mlu_allow_dynamic_smem(band_kernel);
         return v;
     });
@@ -629,8 +686,8 @@ magma_int_t blocked_getrf_steps_l(int m, int n, T **dA, int ldda, int **ipiv, in
     const int pm = m - j0;
     const int rpt = panel_rows_per_thread<T>(pm);
     const size_t smem = rpt == 1   ? panel_regs_smem_bytes<T, 1>()
-                        : rpt == 2 ? panel_regs_smem_bytes<T, 2>()
-                        : rpt == 4 ? panel_regs_smem_bytes<T, (sizeof(T) == 4 ? 4 : 2)>()
+                        : rpt == 2 ? panel_regs_smem_bytes<T, 1, 512>()
+                        : rpt == 4 ? panel_regs_smem_bytes<T, (sizeof(T) == 4 ? 2 : 1), 512>()
                                    : panel_smem_bytes<T>(pm, ib);
     if (!rpt && (smem > PANEL_SMEM_MAX || smem > panel_dyn_max))
         return MAGMA_ERR_NOT_SUPPORTED;   // m too large for a shared-memory panel
@@ -653,14 +710,20 @@ magma_int_t blocked_getrf_steps_l(int m, int n, T **dA, int ldda, int **ipiv, in
         else
             launch_panel<T, false>(rpt, m, n, j0, ib, dAb, ldda, ipb, infb, vs, nb, smem, s);
         const int rm = m - j0 - ib, rn = block_col_end(bj, m, n) - j0 - ib;
-        const int bands = rn > 0 ? (rn + BAND_N - 1) / BAND_N : 0;
+        // columns the grid right of the panel covers: a matrix of a variable-size batch
+        // whose last panel is narrower than ib has up to ib - 1 more of them
+        const int rg = vs.m_arr ? block_col_end(bj, m, n) - j0 - 1 : rn;
+        const int bands = rg > 0 ? (rg + BAND_N - 1) / BAND_N : 0;
         const bool fused = band_used<T>() && update && bands > 0 &&
                            (long long)bands * nb >= (long long)tune.band_ctas * mlu_sm_count();
         const int ncl = defer_left ? 0 : (j0 + SWAP_COLS - 1) / SWAP_COLS;
-        const int ncr = fused ? 0 : (rn + SWAP_COLS - 1) / SWAP_COLS;
-        if (ncl + ncr > 0)
-            MLU_LAUNCH(mlu::KC_SWAP_TRSM, s, swap_trsm_kernel<T><<<dim3(ncl + ncr, nb), SWAP_THREADS, 0, s>>>(
-                m, n, j0, ib, dAb, ldda, ipb, vs, defer_left ? 0 : 1, bj));
+        const int ncr = fused || rg <= 0 ? 0 : (rg + RIGHT_COLS - 1) / RIGHT_COLS;
+        if (ncl > 0 && ipb != nullptr)
+            MLU_LAUNCH(mlu::KC_SWAP_TRSM, s, left_tile_kernel<T><<<dim3(ncl, nb), SWAP_THREADS, 0, s>>>(
+                m, n, j0, ib, dAb, ldda, ipb, vs));
+        if (ncr > 0)
+            MLU_LAUNCH(mlu::KC_SWAP_TRSM, s, right_cols_kernel<T><<<dim3(ncr, nb), RIGHT_COLS, 0, s>>>(
+                m, n, j0, ib, dAb, ldda, ipb, vs, bj));
         if (fused) {
             MLU_LAUNCH(mlu::KC_GEMM, s, band_kernel<<<dim3(bands, nb), BAND_THREADS, band_smem_bytes(), s>>>(
                 m, n, j0, ib, reinterpret_cast<float **>(dAb), ldda, ipb, vs, bj));
@@ -737,6 +800,15 @@ template <typename T>
 static bool outer_blocked(int m, int n)
 {
     return outer_blocked_shape<T>(m, n) && fixed_choice(false, m, n).two_level;
+}
+// ... when its rank-128 updates, one CTA per matrix and 128 columns, give every SM
+// one; below that the one-level steps spread the update over more, smaller CTAs
+// (two-level / one-level, us: n=1000 b=4 2383 / 1810, b=20 2556 / 2505, b=60 3827 /
+// 4246; n=512 b=20 865 / 781, b=60 1012 / 1049; n=300 b=60 520 / 479, b=150 618 / 637).
+template <typename T>
+static bool outer_blocked(int m, int n, int batch)
+{
+    return outer_blocked<T>(m, n) && (long long)batch * mlu_ceildiv(n - OUTER_NB, OUTER_NB) >= mlu_sm_count();
 }
 
 // Steps of the two-level blocked factorisation: per 128-column block, its
@@ -817,7 +889,7 @@ magma_int_t blocked_getrf(int m, int n, T **dA, int ldda, int **ipiv, int *info,
         MLU_CHECK_LAUNCH();
         return MAGMA_SUCCESS;
     }
-    if (outer_blocked<T>(m, n))
+    if (outer_blocked<T>(m, n, batch))
         return blocked_getrf_outer<T>(m, n, dA, ldda, ipiv, info, batch, q, {nullptr, nullptr, nullptr});
     const int mn = min(m, n);
     const bool defer = ipiv != nullptr && m <= LEFT_DEFER_MAX_M;
@@ -867,7 +939,7 @@ magma_int_t blocked_getrf_vbatched(const int *m, const int *n, const int *ld, in
     if (batch <= 0 || max_m <= 0 || max_n <= 0) return MAGMA_SUCCESS;
     const int mn = min(max_m, max_n);
     const StepSizes vs = {m, n, ld};
-    if (outer_blocked<T>(max_m, max_n))
+    if (outer_blocked<T>(max_m, max_n, batch))
         return blocked_getrf_outer<T>(max_m, max_n, dA, 0, ipiv, info, batch, q, vs);
     const bool defer = ipiv != nullptr && max_m <= LEFT_DEFER_MAX_M;
     int panels = 0;

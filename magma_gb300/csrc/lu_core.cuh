@@ -130,7 +130,7 @@ __device__ __forceinline__ int panel_factor(int pm, int ib, T *A, int lda, unsig
                 if (qrow != prow) { sPos[qrow] = P; sRowAt[P] = qrow; }
                 s_prow = prow;
                 s_piv = piv;
-                s_rcp = T(1) / piv;
+                s_rcp = recip(piv);
                 s_ipiv[k] = (int)P;
                 if (!Prec<T>::nonzero(piv) && info_local == 0) info_local = col0 + k + 1;
             }
@@ -187,6 +187,23 @@ __host__ __device__ constexpr size_t panel_regs_smem_bytes()
 {
     return (size_t)PANEL_NB * panel_regs_ld<T, RPT, NT>() * sizeof(T) +
            (size_t)panel_regs_ld<T, RPT, NT>() * sizeof(int);
+}
+
+// The update of a panel row by one step, shifted by one column: a[j - 1] =
+// fma(-l, u_j, a[j]) for the remaining columns 1 <= j < rem (in groups of eight).
+// The guards are nested, so that each encloses enough code to stay a branch: a
+// guarded group by itself is turned into predicated instructions, and an FP64
+// instruction that is predicated off takes its time in the pipe all the same.
+template <typename T, int J>
+__device__ __forceinline__ void panel_shift(T (&a)[PANEL_NB], T l, const T *prow, int rem)
+{
+    if constexpr (J < PANEL_NB) {
+        if (J < rem) {
+#pragma unroll
+            for (int j = J; j < J + 8 && j < PANEL_NB; j++) a[j - 1] = Prec<T>::fma_(-l, prow[j], a[j]);
+            panel_shift<T, J + 8>(a, l, prow, rem);
+        }
+    }
 }
 
 template <typename T, int RPT, bool NOPIV = false, int NT = PANEL_REGS_THREADS>
@@ -274,7 +291,7 @@ __device__ __forceinline__ int panel_factor_regs(int pm, int ib, T *A, int lda, 
 #pragma unroll
         for (int r = 0; r < RPT; r++) any_live |= live[r];
         T rcp = T(0);
-        if (__any_sync(FULL, any_live)) rcp = T(1) / piv;
+        if (__any_sync(FULL, any_live)) rcp = recip(piv);
         if (tid == 0) {
             s_ipiv[k] = (int)gpos;
             if (!nz && info_local == 0) info_local = col0 + k + 1;
@@ -295,18 +312,7 @@ __device__ __forceinline__ int panel_factor_regs(int pm, int ib, T *A, int lda, 
             } else {
                 const T l = nz ? rscale(a[r][0], piv, rcp) : a[r][0];
                 sP[(size_t)k * LDP + slot] = l;
-                // the row's remaining columns are j < ib - k: groups of eight past
-                // them are skipped (the same test in every lane of the block)
-#pragma unroll
-                for (int c = 0; c < PANEL_NB / 8; c++) {
-                    if (8 * c + 1 < ib - k) {
-#pragma unroll
-                        for (int jj = 0; jj < 8; jj++) {
-                            const int j = 8 * c + 1 + jj;
-                            if (j < PANEL_NB) a[r][j - 1] = Prec<T>::fma_(-l, prow[j], a[r][j]);
-                        }
-                    }
-                }
+                panel_shift<T, 1>(a[r], l, prow, ib - k);
             }
         }
     }
@@ -401,54 +407,6 @@ __device__ __forceinline__ void apply_permutation(T *A, int lda, int c0, int c1,
         }
         __syncthreads();
     }
-}
-
-// U12 = L11^{-1} A12 for the columns [c0, c1) of the ib rows starting at row
-// j0 (L11 unit lower, at (j0, j0)), the right-hand sides staged in shared
-// memory (sbuf: PANEL_NB x chunk T): one thread per column, updates
-// u_i = fma(-l_it, u_t, u_i) for t ascending.  All threads call it.
-template <typename T>
-__device__ __forceinline__ void trsm_l11_smem(T *A, int lda, int j0, int ib, int c0, int c1,
-                                              T *sbuf, int chunk)
-{
-    __shared__ T s_L[PANEL_NB][PANEL_NB + 1];
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    for (int e = tid; e < ib * ib; e += nthr) {
-        const int i = e % ib, t = e / ib;
-        s_L[i][t] = A[j0 + i + (size_t)(j0 + t) * lda];
-    }
-    for (int cb = c0; cb < c1; cb += chunk) {
-        const int w = min(chunk, c1 - cb);
-        __syncthreads();
-        const int total = ib * w;
-        for (int e0 = tid; e0 < total; e0 += 8 * nthr) {   // coalesced down each column
-            T v[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int e = e0 + u * nthr;
-                if (e < total) v[u] = A[j0 + e % ib + (size_t)(cb + e / ib) * lda];
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int e = e0 + u * nthr;
-                if (e < total) sbuf[(e % ib) * chunk + e / ib] = v[u];
-            }
-        }
-        __syncthreads();
-        for (int c = tid; c < w; c += nthr) {
-            for (int t = 0; t < ib; t++) {
-                const T ut = sbuf[t * chunk + c];
-                for (int i = t + 1; i < ib; i++)
-                    sbuf[i * chunk + c] = Prec<T>::fma_(-s_L[i][t], ut, sbuf[i * chunk + c]);
-            }
-        }
-        __syncthreads();
-        for (int e = tid; e < ib * w; e += nthr) {
-            const int i = e % ib, c = e / ib;
-            A[j0 + i + (size_t)(cb + c) * lda] = sbuf[i * chunk + c];
-        }
-    }
-    __syncthreads();
 }
 
 // One BM x BN tile of A22 -= L21 * U12 with rows from r0 and columns from c0

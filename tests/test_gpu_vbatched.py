@@ -266,3 +266,30 @@ def test_getrf_vbatched_large_blocked_path(cuda, dtype):
         assert inf[k] == rinfo, k
         assert np.array_equal(A.view(k).cpu().numpy(), ref, equal_nan=True), k
         assert np.array_equal(P[offs[k]:offs[k] + min(m, n)], rp[:min(m, n)]), k
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_getrf_vbatched_wide_with_narrow_last_panels(cuda, dtype):
+    # matrices whose last panel is narrower than the batch's: the columns right of it
+    # reach further than the widest panel's would
+    rng = np.random.default_rng(8)
+    shapes = [(40, 300), (300, 300), (290, 300), (1, 300), (33, 290), (299, 300), (65, 300), (257, 299), (131, 300)]
+    ms, ns = [m for m, _ in shapes], [n for _, n in shapes]
+    td = torch.float64 if dtype == np.float64 else torch.float32
+    As = [rng.uniform(-1, 1, (n, m)).astype(dtype) for m, n in shapes]
+    A = VBatch([a.shape for a in As], ms, td, cuda).load(As)
+    mn = [min(m, n) for m, n in shapes]
+    ipiv = torch.zeros((len(shapes), 300), dtype=torch.int32, device=cuda)
+    dP = ipiv.data_ptr() + torch.arange(len(shapes), dtype=torch.int64, device=cuda) * 300 * 4
+    info = torch.empty((len(shapes),), dtype=torch.int32, device=cuda)
+    q = Queue.current(cuda)
+    f = getattr(L.load(), "magma_dgetrf_vbatched" if dtype == np.float64 else "magma_sgetrf_vbatched")
+    assert f(_vp(A.rows), _vp(A.ncols), _vp(A.ptrs), _vp(A.ld), _vp(dP), _vp(info), len(shapes), q.handle) == 0
+    torch.cuda.synchronize()
+    g = oracle.dgetrf_batched if dtype == np.float64 else oracle.sgetrf_batched
+    P = ipiv.cpu().numpy()
+    for k, (m, n) in enumerate(shapes):
+        r = As[k][None].copy()
+        rp, ri = g(r, m)
+        assert np.array_equal(P[k, :mn[k]], rp[0, :mn[k]]), k
+        assert np.array_equal(A.view(k).cpu().numpy(), r[0]), k
