@@ -125,7 +125,7 @@ left_tile_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ipi
 // (one FP64 warp instruction per 64 cycles and scheduler), FP32 by the latency of
 // the loads.  n = 512 FP64, 512 matrices: the form with one tile of columns in shared
 // memory (two of four warps solving) took 4260 us per factorisation, this one
-// RIGHT_US; n = 1000 FP32, six matrices: 36 us a step, now RIGHT32_US.
+// 3150; n = 1000 FP32, six matrices: 36 us a step, now 12.
 constexpr int RIGHT_COLS = 64;
 
 template <typename T>
