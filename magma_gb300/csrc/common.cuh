@@ -80,11 +80,15 @@ static __device__ __noinline__ double div_call(double a, double b) { return a / 
 // remainder 2^105 - q m decides the last bit; 2^106 = (2q + 1) m has no solution
 // but for powers of two, so there are no ties.  Zero, subnormal, infinite and
 // NaN operands, and those whose reciprocal is subnormal, take the division.
-__device__ __forceinline__ double recip(double x)
+// recip_plain: without the test for those operands (recip_special), branch-free.
+__device__ __forceinline__ bool recip_special(double x)
+{
+    return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 1u > 2043u;
+}
+__device__ __forceinline__ double recip_plain(double x)
 {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const unsigned e = (hi >> 20) & 0x7ffu;
-    if (e - 1u > 2043u) return div_call(1.0, x);
     const unsigned mh = (hi & 0xfffffu) | 0x100000u;                  // m = mh:lo, 53 bits
     const unsigned d1 = __funnelshift_l(lo, mh, 11), d0 = lo << 11;   // m << 11
     float y;
@@ -109,6 +113,9 @@ __device__ __forceinline__ double recip(double x)
     const unsigned long long b = q + ((unsigned long long)(2044u - e) << 52);
     return __longlong_as_double((long long)(b | ((unsigned long long)(hi & 0x80000000u) << 32)));
 }
+__device__ __forceinline__ double recip(double x) { return recip_special(x) ? div_call(1.0, x) : recip_plain(x); }
+__device__ __forceinline__ bool recip_special(float) { return false; }
+__device__ __forceinline__ float recip_plain(float x) { return 1.f / x; }
 __device__ __forceinline__ float recip(float x) { return 1.f / x; }
 
 // x scaled by the reciprocal r of d, or divided by d when d is subnormal

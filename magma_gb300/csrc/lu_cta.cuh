@@ -45,6 +45,7 @@ __host__ __device__ constexpr size_t cta_lu_smem(int max_m, int max_n)
 // row, the current column first.
 template <typename T> struct CtaPanel {
     T rest[2][8][CTA_NB];
+    T rcp[2][8];             // reciprocal of rest[..][0] (not valid where recip_special)
     T top[CTA_NB][CTA_NB];   // U rows of the panel
     unsigned hi[2][8], lo[2][8], pos[2][8];
     int ipiv[CTA_NB];        // position chosen at each column
@@ -52,40 +53,58 @@ template <typename T> struct CtaPanel {
     int dst[CTA_NB];         // original top row i goes to this row (-1: it stays in the top block)
 };
 
-// The update of a panel row by one step, shifted by one column: a[j - 1] =
-// fma(-l, u_j, a[j]) for the columns 1 <= j < REM, u_j at rest[j].
+// One step's update of a panel row and the search of the next column.  a[j - 1] =
+// fma(-l, u_j, a[j]) for 1 <= j < REM (u_j at rest[j]): shifted, so that the current
+// column stays a[0]; then the warp's best candidate of that column, published with
+// its reciprocal for step k + 1.  Straight-line: the search and the reciprocal are
+// integer instructions on the new a[0] alone, which is computed first, and issue
+// between the other FMAs, 64 cycles apart on the FP64 pipe.  REM <= 1: no update
+// (before the first step).  Rows already chosen as pivots go through the motions.
 template <typename T, int REM>
-__device__ __forceinline__ void cta_shift_update(T (&a)[CTA_NB], T l, const T *rest)
+__device__ __forceinline__ void cta_step(T (&a)[CTA_NB], T l, const T *rest, CtaPanel<T> &s, int buf, int chunk,
+                                         bool live, int pos, int k)
 {
+    if (REM > 1) a[0] = Prec<T>::fma_(-l, rest[1], a[1]);
+    unsigned long long mag = Prec<T>::absbits(a[0]);
+    if (Prec<T>::isnan_(a[0])) mag = pos == k ? 0x7fffffffffffffffull : 0ull;
+    const unsigned long long key = live ? mag | 0x8000000000000000ull : 0ull;
+    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+    const unsigned mhi = __reduce_max_sync(FULL, hi);
+    const unsigned mlo = __reduce_max_sync(FULL, hi == mhi ? lo : 0u);
+    const unsigned mp = __reduce_min_sync(FULL, live && hi == mhi && lo == mlo ? (unsigned)pos : 0xffffffffu);
+    const bool win = live && (unsigned)pos == mp;
+    const T r = recip_plain(a[0]);                       // (the winner's is used)
 #pragma unroll
-    for (int j = 1; j < REM; j++) a[j - 1] = Prec<T>::fma_(-l, rest[j], a[j]);
+    for (int j = 2; j < REM; j++) a[j - 1] = Prec<T>::fma_(-l, rest[j], a[j]);
+    if (win) {
+        s.hi[buf][chunk] = mhi;
+        s.lo[buf][chunk] = mlo;
+        s.pos[buf][chunk] = mp;
+        s.rcp[buf][chunk] = r;
+#pragma unroll
+        for (int j = 0; j < (REM > 1 ? REM - 1 : CTA_NB); j++) s.rest[buf][chunk][j] = a[j];
+    }
+    if (mhi == 0u && (threadIdx.x & 31) == 0) s.hi[buf][chunk] = 0u;   // no row left in this block
 }
 
-// ... for rem columns: a jump to straight-line code.  Guards (j < rem) would be
-// turned into predicates, and an FP64 instruction that is predicated off takes
-// its full 16 cycles of the pipe (panel of 64 rows, twelve CTAs per SM: 153,000
-// cycles with guards).
+// ... with rem columns remaining at the step: a jump to the code for that many,
+// rounded up to even.  Guards (j < rem) would be turned into predicates, and an
+// FP64 instruction that is predicated off takes its full 16 cycles of the pipe
+// (panel of 64 rows, twelve CTAs per SM: 153,000 cycles with guards).
 template <typename T>
-__device__ __forceinline__ void cta_shift_update(T (&a)[CTA_NB], T l, const T *rest, int rem)
+__device__ __forceinline__ void cta_step(T (&a)[CTA_NB], T l, const T *rest, CtaPanel<T> &s, int buf, int chunk,
+                                         bool live, int pos, int k, int rem)
 {
     static_assert(CTA_NB == 16, "cases");
-    switch (rem) {
-    case 2: cta_shift_update<T, 2>(a, l, rest); break;
-    case 3: cta_shift_update<T, 3>(a, l, rest); break;
-    case 4: cta_shift_update<T, 4>(a, l, rest); break;
-    case 5: cta_shift_update<T, 5>(a, l, rest); break;
-    case 6: cta_shift_update<T, 6>(a, l, rest); break;
-    case 7: cta_shift_update<T, 7>(a, l, rest); break;
-    case 8: cta_shift_update<T, 8>(a, l, rest); break;
-    case 9: cta_shift_update<T, 9>(a, l, rest); break;
-    case 10: cta_shift_update<T, 10>(a, l, rest); break;
-    case 11: cta_shift_update<T, 11>(a, l, rest); break;
-    case 12: cta_shift_update<T, 12>(a, l, rest); break;
-    case 13: cta_shift_update<T, 13>(a, l, rest); break;
-    case 14: cta_shift_update<T, 14>(a, l, rest); break;
-    case 15: cta_shift_update<T, 15>(a, l, rest); break;
-    case 16: cta_shift_update<T, 16>(a, l, rest); break;
-    default: break;
+    switch ((rem + 1) >> 1) {
+    case 1: cta_step<T, 2>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 2: cta_step<T, 4>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 3: cta_step<T, 6>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 4: cta_step<T, 8>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 5: cta_step<T, 10>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 6: cta_step<T, 12>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 7: cta_step<T, 14>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    default: cta_step<T, 16>(a, l, rest, s, buf, chunk, live, pos, k); break;
     }
 }
 
@@ -96,9 +115,8 @@ __device__ __forceinline__ void cta_shift_update(T (&a)[CTA_NB], T l, const T *r
 // first zero pivot, or 0, in every thread with a row.
 //
 // A row's remaining columns sit in its thread's registers with the current one
-// first: the update of step k writes column j into a[j - 1], so that the column
-// loop stays a loop (its code is run 16 times, not once).  A column that is done
-// leaves for sP, in physical row order until the end.
+// first, so that the column loop stays a loop.  A column that is done leaves for
+// sP, in physical row order until the end.
 template <typename T>
 __device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, int ldp, CtaPanel<T> &s, int i)
 {
@@ -110,70 +128,46 @@ __device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, 
     T a[CTA_NB];
 #pragma unroll
     for (int j = 0; j < CTA_NB; j++) a[j] = row && j < ib ? Ap[i + (size_t)j * lda] : T(0);
+    if (chunk < nch) cta_step<T, 1>(a, T(0), nullptr, s, 0, chunk, live, pos, 0);
 #pragma unroll 1
     for (int k = 0; k < ib; k++) {
         const int buf = k & 1;
-        if (chunk < nch) {
-            unsigned long long key = 0ull;
-            if (live) {
-                unsigned long long mag = Prec<T>::absbits(a[0]);
-                if (Prec<T>::isnan_(a[0])) mag = pos == k ? 0x7fffffffffffffffull : 0ull;
-                key = mag | 0x8000000000000000ull;
-            }
-            const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-            const unsigned mhi = __reduce_max_sync(FULL, hi);
-            unsigned win = __ballot_sync(FULL, live && hi == mhi);
-            if (win & (win - 1)) {                       // upper halves tie: the lower, then the positions
-                const unsigned mlo = __reduce_max_sync(FULL, hi == mhi ? lo : 0u);
-                const bool c = live && hi == mhi && lo == mlo;
-                const unsigned mp = __reduce_min_sync(FULL, c ? (unsigned)pos : 0xffffffffu);
-                win = __ballot_sync(FULL, c && (unsigned)pos == mp);
-            }
-            if ((win >> lane) & 1) {
-                s.lo[buf][chunk] = lo;
-                s.pos[buf][chunk] = (unsigned)pos;
-#pragma unroll
-                for (int j = 0; j < CTA_NB; j++) s.rest[buf][chunk][j] = a[j];
-            }
-            if (lane == 0) s.hi[buf][chunk] = mhi;
-        }
         if (nch > 1) __syncthreads();
         else __syncwarp();
-        if (chunk < nch) {
-            int gw = 0;
-            if (nch > 1) {
-                const unsigned h = lane < nch ? s.hi[buf][lane] : 0u;
-                const unsigned mh = __reduce_max_sync(FULL, h);
-                unsigned eq = __ballot_sync(FULL, lane < nch && h == mh);
-                if (eq & (eq - 1)) {                     // the upper halves tie: the lower, then the positions
-                    const bool c = (eq >> lane) & 1;
-                    const unsigned l = c ? s.lo[buf][lane] : 0u;
-                    const unsigned ml = __reduce_max_sync(FULL, l);
-                    const unsigned p = c && l == ml ? s.pos[buf][lane] : 0xffffffffu;
-                    const unsigned mp = __reduce_min_sync(FULL, p);
-                    eq = __ballot_sync(FULL, c && p == mp);
-                }
-                gw = __ffs(eq) - 1;
+        if (chunk >= nch) continue;
+        int gw = 0;
+        if (nch > 1) {
+            const unsigned h = lane < nch ? s.hi[buf][lane] : 0u;
+            const unsigned mh = __reduce_max_sync(FULL, h);
+            unsigned eq = __ballot_sync(FULL, lane < nch && h == mh);
+            if (eq & (eq - 1)) {                         // the upper halves tie: the lower, then the positions
+                const bool c = (eq >> lane) & 1;
+                const unsigned l = c ? s.lo[buf][lane] : 0u;
+                const unsigned ml = __reduce_max_sync(FULL, l);
+                const unsigned p = c && l == ml ? s.pos[buf][lane] : 0xffffffffu;
+                const unsigned mp = __reduce_min_sync(FULL, p);
+                eq = __ballot_sync(FULL, c && p == mp);
             }
-            const unsigned gpos = s.pos[buf][gw];
-            const T piv = s.rest[buf][gw][0];
-            const bool nz = Prec<T>::nonzero(piv);
-            if (!nz && info == 0) info = k + 1;
-            if (i == 0) s.ipiv[k] = (int)gpos;
-            const T r = recip(piv);
-            if (chunk == 0 && lane < ib - k) s.top[k][k + lane] = s.rest[buf][gw][lane];
-            if (pos == (int)gpos) {
-                live = false;                            // the pivot row is U row k
-                pos = k;
-            } else if (pos == k) {
-                pos = (int)gpos;
-            }
-            if (live) {
-                const T l = nz ? rscale(a[0], piv, r) : a[0];
-                sP[k * ldp + i] = l;
-                cta_shift_update<T>(a, l, s.rest[buf][gw], ib - k);
-            }
+            gw = __ffs(eq) - 1;
         }
+        const T *rest = s.rest[buf][gw];
+        const unsigned gpos = s.pos[buf][gw];
+        const T piv = rest[0];
+        T r = s.rcp[buf][gw];
+        const bool nz = Prec<T>::nonzero(piv);
+        if (!nz && info == 0) info = k + 1;
+        if (i == 0) s.ipiv[k] = (int)gpos;
+        if (chunk == 0 && lane < ib - k) s.top[k][k + lane] = rest[lane];
+        if (pos == (int)gpos) {
+            live = false;                                // the pivot row is U row k
+            pos = k;
+        } else if (pos == k) {
+            pos = (int)gpos;
+        }
+        T l = a[0] * r;
+        if (recip_special(piv)) l = nz ? rscale(a[0], piv, recip(piv)) : a[0];
+        if (row) sP[k * ldp + i] = l;                    // (rows already chosen: never read)
+        if (k + 1 < ib) cta_step<T>(a, l, rest, s, buf ^ 1, chunk, live, pos, k + 1, ib - k);
     }
     // pivoted order: every row to its position, in shared memory and in A.  A row's
     // L entries are its own stores (no barrier needed to read them back); a top row
