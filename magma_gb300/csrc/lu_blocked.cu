@@ -714,7 +714,11 @@ magma_int_t blocked_getrf_steps_l(int m, int n, T **dA, int ldda, int **ipiv, in
         // whose last panel is narrower than ib has up to ib - 1 more of them
         const int rg = vs.m_arr ? block_col_end(bj, m, n) - j0 - 1 : rn;
         const int bands = rg > 0 ? (rg + BAND_N - 1) / BAND_N : 0;
-        const bool fused = band_used<T>() && update && bands > 0 &&
+        // The fused band kernel pays for its set-up (five barriers, two CTAs per SM) on
+        // long columns only: batch 1000, getrf us with it / with the separate kernels,
+        // two-level n=200 1204 / 1065, n=320 2708 / 2647, n=512 6274 / 6303;
+        // one-level n=256 1868 / 1810, n=320 3030 / 3145, n=512 8557 / 9943.
+        const bool fused = band_used<T>() && update && bands > 0 && max(m, n) > (bj < 0 ? 288 : 384) &&
                            (long long)bands * nb >= (long long)tune.band_ctas * mlu_sm_count();
         const int ncl = defer_left ? 0 : (j0 + SWAP_COLS - 1) / SWAP_COLS;
         const int ncr = fused || rg <= 0 ? 0 : (rg + RIGHT_COLS - 1) / RIGHT_COLS;
@@ -804,11 +808,13 @@ static bool outer_blocked(int m, int n)
 // ... when its rank-128 updates, one CTA per matrix and 128 columns, give every SM
 // one; below that the one-level steps spread the update over more, smaller CTAs
 // (two-level / one-level, us: n=1000 b=4 2383 / 1810, b=20 2556 / 2505, b=60 3827 /
-// 4246; n=512 b=20 865 / 781, b=60 1012 / 1049; n=300 b=60 520 / 479, b=150 618 / 637).
+// 4246; n=512 b=20 865 / 781, b=60 1012 / 1049; n=300 b=60 520 / 479, b=150 618 / 637),
+// and when enough columns lie right of the first block (b=1000: n=144 732 / 572,
+// n=200 1065 / 1153).
 template <typename T>
 static bool outer_blocked(int m, int n, int batch)
 {
-    return outer_blocked<T>(m, n) && (long long)batch * mlu_ceildiv(n - OUTER_NB, OUTER_NB) >= mlu_sm_count();
+    return outer_blocked<T>(m, n) && n > 176 && (long long)batch * mlu_ceildiv(n - OUTER_NB, OUTER_NB) >= mlu_sm_count();
 }
 
 // Steps of the two-level blocked factorisation: per 128-column block, its
