@@ -114,7 +114,8 @@ __device__ __forceinline__ double recip_plain(double x)
     return __longlong_as_double((long long)(b | ((unsigned long long)(hi & 0x80000000u) << 32)));
 }
 __device__ __forceinline__ double recip(double x) { return recip_special(x) ? div_call(1.0, x) : recip_plain(x); }
-__device__ __forceinline__ bool recip_special(float) { return false; }
+// FP32: 1/x is right for every operand; a zero or subnormal one is not to be multiplied by it
+__device__ __forceinline__ bool recip_special(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0u; }
 __device__ __forceinline__ float recip_plain(float x) { return 1.f / x; }
 __device__ __forceinline__ float recip(float x) { return 1.f / x; }
 

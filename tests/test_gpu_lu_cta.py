@@ -14,22 +14,23 @@ pytestmark = pytest.mark.gpu
 BATCH = 160          # one CTA per matrix needs a batch that occupies the SMs
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("m,n", [(33, 33), (48, 48), (49, 49), (63, 63), (64, 64), (65, 65), (97, 97), (128, 128),
                                  (129, 129), (160, 160), (255, 255), (256, 256), (256, 40), (40, 256), (7, 200),
                                  (200, 7), (130, 65)])
-def test_getrf_one_cta_per_matrix(cuda, m, n):
+def test_getrf_one_cta_per_matrix(cuda, m, n, dtype):
     rng = np.random.default_rng(m * 7 + n)
     k = 10
-    A = rng.uniform(-1, 1, (k, m, n))
+    A = rng.uniform(-1, 1, (k, m, n)).astype(dtype)
     A[1, :, min(m, n) // 2] = 0.0                 # a zero column
     A[2] = rng.integers(-2, 3, (m, n))            # ties in the pivot search
     A[3, m // 2, :] = np.nan
     A[4, :, 0] = np.inf
-    A[5] *= 1e-310                                # subnormal pivots
+    A[5] *= dtype(1e-310 if dtype == np.float64 else 1e-40)      # subnormal pivots
     S = to_storage(A, m + 3)
     S[:, :, m:] = 9.0
     rS = S.copy()
-    ripiv, rinfo = oracle.dgetrf_batched(rS, m)
+    ripiv, rinfo = (oracle.dgetrf_batched if dtype == np.float64 else oracle.sgetrf_batched)(rS, m)
     dS = torch.from_numpy(np.ascontiguousarray(S[np.arange(BATCH) % k])).to(cuda)
     ipiv, info = mg.getrf_batched(dS, m)
     torch.cuda.synchronize()
