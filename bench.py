@@ -127,7 +127,7 @@ class Gesv32:
             raise RuntimeError(f"magma_dgesv_batched returned {rc}")
 
     dominant_class = "small_gesv"
-    dominant = "mlu::small_gesv_kernel<double,32,1>"
+    dominant = "mlu::small_gesv_packed_kernel<double>"
 
     # End to end: two calls on the two halves of the batch; the second half's host-to-device
     # copy runs on a copy stream while the first half is solved, and each half's solutions
@@ -1248,7 +1248,7 @@ TRAFFIC = {
                 "matrix-passes, scaled by the residual passes of the step "
                 "(profiles/ir_residual_kernel_fp64_n512_batch128.md)"},
     "gesv32": {
-        "kernel": "mlu::small_gesv_kernel<double,32,1>", "unit": "matrix (n=32, nrhs=1)",
+        "kernel": "mlu::small_gesv_packed_kernel<double>", "unit": "matrix (n=32, nrhs=1)",
         "dram_bytes_per_unit": 110.8e6 / 10000,
         "note": "ncu capture of one launch over 10,000 matrices: 84.9 MB read + 25.8 MB written "
                 "(profiles/small_gesv_kernel_fp64_n32_batch10000.md)"},

@@ -629,16 +629,19 @@ static void launch_panel(int rpt, int m, int n, int j0, int ib, T **dA, int ldda
 }
 
 // The whole factorisation of a matrix of at most NT rows and columns by one CTA
-// of NT threads (lu_cta.cuh); dynamic shared memory cta_lu_smem.
+// of NT threads (lu_cta.cuh); dynamic shared memory cta_lu_smem.  FP64: as many CTAs
+// per SM as 72 registers a thread allow, for what is left of a batch after the full
+// waves (n = 100, seven matrices per SM: 1012 us with six CTAs, 859 now; n = 64,
+// 13: 519, 466).  FP32 loses by it (n = 40, 1500 matrices: 61 us, 66).
 template <typename T, int NT>
-__global__ void __launch_bounds__(NT, 768 / NT)
+__global__ void __launch_bounds__(NT, (sizeof(T) == 8 ? 896 : 768) / NT)
 lu_cta_kernel(int m, int n, T **dA_array, int ldda, int **ipiv_array, int *info_array)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ __align__(16) CtaPanel<T> s_panel;
+    __shared__ __align__(16) CtaPanel<T, NT / 32> s_panel;
     const int mat = blockIdx.x;
-    cta_lu<T>(m, n, dA_array[mat], ldda, ipiv_array[mat], 0, nullptr, 1, smem_raw, cta_ld(m), cta_ld(n), s_panel, CTA_NB,
-              false, cta_rot(mat), &info_array[mat]);
+    cta_lu<T>(m, n, dA_array[mat], ldda, ipiv_array[mat], 0, nullptr, 1, smem_raw, cta_ldp(m), cta_ldu(n, min(m, CTA_NB)),
+              s_panel, CTA_NB, false, cta_rot(mat), &info_array[mat]);
 }
 
 template <typename T, int NT>
@@ -646,9 +649,8 @@ static void launch_lu_cta(int m, int n, T **dA, int ldda, int **ipiv, int *info,
 {
     static size_t dyn_cache[MLU_MAX_DEVICES];
     mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(lu_cta_kernel<T, NT>); });
-    MLU_LAUNCH(mlu::KC_PANEL, s, lu_cta_kernel<T, NT><<<batch, NT, cta_lu_smem<T>(m, n), s>>>(m, n, dA, ldda, ipiv, info));
+    MLU_LAUNCH(mlu::KC_PANEL, s, lu_cta_kernel<T, NT><<<batch, NT, cta_lu_smem<T>(m, n, min(m, CTA_NB)), s>>>(m, n, dA, ldda, ipiv, info));
 }
-
 
 // One step of the blocked factorisation for every matrix: panel at column j0
 // of width ib, interchanges + TRSM, and (when `update`) the trailing update.
@@ -866,21 +868,22 @@ static magma_int_t blocked_getrf_outer(int m, int n, T **dA, int ldda, int **ipi
 // Whether the one-CTA kernel (lu_cta.cuh) takes a batch whose larger dimension is
 // n, or the step kernels, which spread a matrix over many CTAs.  Measured per call
 // (step kernels / one CTA, us):
-//   FP64 n=64:  b=8 242 / 222, b=1500 605 / 442;  n=128: b=8 546 / 527, b=1500 3039 / 2198
-//        n=160: b=8 697 / 714, b=76 773 / 718;    n=200: b=8 970 / 1157, b=76 1274 / 1161
-//        n=256: b=76 1753 / 2024, b=152 2407 / 2044, b=1500 18235 / 15777
-//   FP32 n=64:  b=8 163 / 152, b=1500 270 / 208;  n=128: b=8 299 / 271, b=1500 747 / 740
-//        n=200: b=8 480 / 443, b=300 586 / 519, b=600 814 / 1012;  n=256: b=8 574 / 679
-// FP64 is bound by its pipe, which one CTA per SM fills for large orders: above 128
-// the batch has to occupy the SMs.  FP32 above 128 is the other way round: the
-// register-blocked rank-128 updates win once there are two matrices per SM.
+//   FP64 n=64:  b=4 146 / 144, b=1000 279 / 281, b=3000 740 / 679
+//        n=80:  b=4 222 / 175, b=3000 1633 / 1258;  n=112: b=4 341 / 337, b=3000 4088 / 2797
+//        n=128: b=4 380 / 431, b=76 414 / 435, b=100 449 / 437, b=152 480 / 437, b=3000 4771 / 3965
+//        n=160: b=8 497 / 599, b=76 570 / 603, b=152 715 / 607, b=1500 4527 / 3867
+//        n=200: b=8 699 / 1035, b=76 996 / 1041, b=152 1389 / 1043, b=1500 9807 / 7347
+//        n=256: b=8 890 / 1875, b=76 1440 / 1885, b=152 2113 / 1903, b=1500 16641 / 15228
+//   FP32 n=33:  b=4 54 / 44, b=3000 134 / 105;   n=48: b=4 60 / 52, b=3000 166 / 136
+//        n=52:  b=4 62 / 66, b=3000 175 / 191;   n=128: b=8 149 / 187, b=1500 531 / 651
+// FP64 is bound by its pipe, which the one-CTA kernel wastes less of once there is
+// about a matrix per SM.  FP32 is bound by the steps' latency, and a 32-column panel
+// of the step kernels has half as many steps outside it.
 template <typename T>
 static bool one_cta_per_matrix(int n, int batch)
 {
-    if (n > CTA_MAX_N) return false;
-    if (n <= 128) return true;
-    if (sizeof(T) == 8) return (long long)batch * 152 >= (long long)(n - 128) * mlu_sm_count();
-    return n <= 208 && batch <= 2 * mlu_sm_count();
+    if (sizeof(T) == 4) return n <= 48;
+    return n <= 112 || (n <= CTA_MAX_N && 4LL * batch >= 3LL * mlu_sm_count());
 }
 
 template <typename T>
@@ -889,9 +892,11 @@ magma_int_t blocked_getrf(int m, int n, T **dA, int ldda, int **ipiv, int *info,
 {
     if (batch <= 0 || m == 0 || n == 0) return MAGMA_SUCCESS;
     if (ipiv != nullptr && one_cta_per_matrix<T>(max(m, n), batch)) {
-        if (max(m, n) <= 64) launch_lu_cta<T, 64>(m, n, dA, ldda, ipiv, info, batch, q->stream);
-        else if (max(m, n) <= 128) launch_lu_cta<T, 128>(m, n, dA, ldda, ipiv, info, batch, q->stream);
-        else launch_lu_cta<T, 256>(m, n, dA, ldda, ipiv, info, batch, q->stream);
+        if (sizeof(T) == 4 || max(m, n) <= 64) launch_lu_cta<T, 64>(m, n, dA, ldda, ipiv, info, batch, q->stream);
+        else if constexpr (sizeof(T) == 8) {
+            if (max(m, n) <= 128) launch_lu_cta<T, 128>(m, n, dA, ldda, ipiv, info, batch, q->stream);
+            else launch_lu_cta<T, 256>(m, n, dA, ldda, ipiv, info, batch, q->stream);
+        }
         MLU_CHECK_LAUNCH();
         return MAGMA_SUCCESS;
     }
@@ -968,7 +973,11 @@ template magma_int_t blocked_getrf_vbatched<float>(const int *, const int *, con
 
 // ---------------------------------------------------------------------------
 // Blocked solves.  One CTA per (matrix, group of nc right-hand sides) runs the
-// two triangular sweeps of solve_core.cuh on them in shared memory.
+// two triangular sweeps of solve_core.cuh on them in shared memory.  FP64 is bound
+// by its pipe (500 matrices of order 150 with 16 right-hand sides, N / T: 1148 /
+// 830 us with each diagonal block on one warp, 461 / 477 now, 286 at the pipe's
+// peak), FP32 by instruction issue (1000 of order 200 with 8: 436 us, 196 now; the
+// factors are read in 24).
 
 constexpr int SOLVE_THREADS = 256;
 constexpr int SOLVE_NC = 8;                // right-hand sides per CTA, at most

@@ -8,7 +8,7 @@
 // for 16 cycles (one scheduler's share for 64) however many of its lanes work,
 // so every phase is laid out to fill its lanes and to keep warps of all four
 // schedulers busy, and the serial parts of one matrix run beside the updates
-// of the other CTAs of the SM (three of 256 threads, six of 128, twelve of 64):
+// of the other CTAs of the SM (three of 256 threads, seven of 128, fourteen of 64):
 //   panel   CTA_NB columns in registers, a row per thread, rows in place; one
 //           barrier per column; the reciprocal on the integer pipes (recip);
 //   columns one thread per column outside the panel and per right-hand side:
@@ -20,8 +20,8 @@
 //           from shared memory, the blocks dealt out to lanes in one sequence,
 //           so that no lane is idle but in the last group of 32.
 // Panels are 16 columns wide: A22 goes through registers once per 16 steps,
-// which the caches serve beside the FP64 pipe, and the panel and U12 (33 KB
-// each at order 256) leave room for three CTAs.
+// which the caches serve beside the FP64 pipe, and the panel and U12 (63 KB
+// together at order 256, 16 at order 64) leave room for those CTAs.
 #pragma once
 #include "common.cuh"
 
@@ -30,24 +30,26 @@ namespace mlu {
 constexpr int CTA_NB = 16;
 constexpr int CTA_MAX_N = 256;
 
-// Row strides of the panel and of U12 in shared memory: a multiple of four
-// elements with room for a 4 x 4 block that crosses the matrix's edge.
-__host__ __device__ constexpr int cta_ld(int n) { return ((n + 3) & ~3) + 4; }
+// Row strides in shared memory, multiples of four elements (a 4 x 4 block reads up
+// to there): of the panel, and of U12 after a first panel of nb columns or more, whose
+// place also holds the panel's U rows while it is factored.  No more than that:
+// the CTAs per SM depend on it.
+__host__ __device__ constexpr int cta_ldp(int m) { return (m + 3) & ~3; }
+__host__ __device__ constexpr int cta_ldu(int n, int nb) { return n - nb > CTA_NB ? (n - nb + 3) & ~3 : CTA_NB; }
 template <typename T>
-__host__ __device__ constexpr size_t cta_lu_smem(int max_m, int max_n)
+__host__ __device__ constexpr size_t cta_lu_smem(int max_m, int max_n, int nb)
 {
-    return (size_t)CTA_NB * (cta_ld(max_m) + cta_ld(max_n)) * sizeof(T);
+    return (size_t)CTA_NB * (cta_ldp(max_m) + cta_ldu(max_n, nb)) * sizeof(T);
 }
 
 // Shared state of one panel.  Each 32-row block (one warp) publishes its best
 // candidate of the current column, double-buffered: |v| as a 63-bit key (NaN by
 // idamax's rule), its position (ties go to the smaller) and what remains of its
-// row, the current column first.
-template <typename T> struct CtaPanel {
-    T rest[2][8][CTA_NB];
-    T rcp[2][8];             // reciprocal of rest[..][0] (not valid where recip_special)
-    T top[CTA_NB][CTA_NB];   // U rows of the panel
-    unsigned hi[2][8], lo[2][8], pos[2][8];
+// row, the current column first.  NCH: 32-row blocks, at most.
+template <typename T, int NCH> struct CtaPanel {
+    T rest[2][NCH][CTA_NB];
+    T rcp[2][NCH];           // reciprocal of rest[..][0] (not valid where recip_special)
+    unsigned hi[2][NCH], lo[2][NCH], pos[2][NCH];
     int ipiv[CTA_NB];        // position chosen at each column
     int slot[CTA_NB];        // top row q comes from this row
     int dst[CTA_NB];         // original top row i goes to this row (-1: it stays in the top block)
@@ -60,8 +62,8 @@ template <typename T> struct CtaPanel {
 // integer instructions on the new a[0] alone, which is computed first, and issue
 // between the other FMAs, 64 cycles apart on the FP64 pipe.  REM <= 1: no update
 // (before the first step).  Rows already chosen as pivots go through the motions.
-template <typename T, int REM>
-__device__ __forceinline__ void cta_step(T (&a)[CTA_NB], T l, const T *rest, CtaPanel<T> &s, int buf, int chunk,
+template <int REM, typename T, int NCH>
+__device__ __forceinline__ void cta_step(T (&a)[CTA_NB], T l, const T *rest, CtaPanel<T, NCH> &s, int buf, int chunk,
                                          bool live, int pos, int k)
 {
     if (REM > 1) a[0] = Prec<T>::fma_(-l, rest[1], a[1]);
@@ -91,20 +93,20 @@ __device__ __forceinline__ void cta_step(T (&a)[CTA_NB], T l, const T *rest, Cta
 // rounded up to even.  Guards (j < rem) would be turned into predicates, and an
 // FP64 instruction that is predicated off takes its full 16 cycles of the pipe
 // (panel of 64 rows, twelve CTAs per SM: 153,000 cycles with guards).
-template <typename T>
-__device__ __forceinline__ void cta_step(T (&a)[CTA_NB], T l, const T *rest, CtaPanel<T> &s, int buf, int chunk,
+template <typename T, int NCH>
+__device__ __forceinline__ void cta_step(T (&a)[CTA_NB], T l, const T *rest, CtaPanel<T, NCH> &s, int buf, int chunk,
                                          bool live, int pos, int k, int rem)
 {
     static_assert(CTA_NB == 16, "cases");
     switch ((rem + 1) >> 1) {
-    case 1: cta_step<T, 2>(a, l, rest, s, buf, chunk, live, pos, k); break;
-    case 2: cta_step<T, 4>(a, l, rest, s, buf, chunk, live, pos, k); break;
-    case 3: cta_step<T, 6>(a, l, rest, s, buf, chunk, live, pos, k); break;
-    case 4: cta_step<T, 8>(a, l, rest, s, buf, chunk, live, pos, k); break;
-    case 5: cta_step<T, 10>(a, l, rest, s, buf, chunk, live, pos, k); break;
-    case 6: cta_step<T, 12>(a, l, rest, s, buf, chunk, live, pos, k); break;
-    case 7: cta_step<T, 14>(a, l, rest, s, buf, chunk, live, pos, k); break;
-    default: cta_step<T, 16>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 1: cta_step<2>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 2: cta_step<4>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 3: cta_step<6>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 4: cta_step<8>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 5: cta_step<10>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 6: cta_step<12>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    case 7: cta_step<14>(a, l, rest, s, buf, chunk, live, pos, k); break;
+    default: cta_step<16>(a, l, rest, s, buf, chunk, live, pos, k); break;
     }
 }
 
@@ -112,13 +114,15 @@ __device__ __forceinline__ void cta_step(T (&a)[CTA_NB], T l, const T *rest, Cta
 // `i` (a permutation of the thread index by whole warps) per thread.  On return
 // sP[j * ldp + i] and Ap hold it in pivoted order, s.ipiv / slot / dst are set
 // (visible to all threads) and the return value is the 1-based column of the
-// first zero pivot, or 0, in every thread with a row.
+// first zero pivot, or 0, in every thread with a row.  top: room for the panel's U rows
+// (volatile: without it the bounds-check build, which is relocatable code, came out of
+// the compiler with one column of the first update taken from another).
 //
 // A row's remaining columns sit in its thread's registers with the current one
 // first, so that the column loop stays a loop.  A column that is done leaves for
 // sP, in physical row order until the end.
-template <typename T>
-__device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, int ldp, CtaPanel<T> &s, int i)
+template <typename T, int NCH>
+__device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, int ldp, volatile T *top, CtaPanel<T, NCH> &s, int i)
 {
     const int lane = i & 31, chunk = i >> 5;
     const int nch = (pm + 31) >> 5;                      // 32-row blocks
@@ -128,7 +132,7 @@ __device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, 
     T a[CTA_NB];
 #pragma unroll
     for (int j = 0; j < CTA_NB; j++) a[j] = row && j < ib ? Ap[i + (size_t)j * lda] : T(0);
-    if (chunk < nch) cta_step<T, 1>(a, T(0), nullptr, s, 0, chunk, live, pos, 0);
+    if (chunk < nch) cta_step<1>(a, T(0), (const T *)nullptr, s, 0, chunk, live, pos, 0);
 #pragma unroll 1
     for (int k = 0; k < ib; k++) {
         const int buf = k & 1;
@@ -157,7 +161,7 @@ __device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, 
         const bool nz = Prec<T>::nonzero(piv);
         if (!nz && info == 0) info = k + 1;
         if (i == 0) s.ipiv[k] = (int)gpos;
-        if (chunk == 0 && lane < ib - k) s.top[k][k + lane] = rest[lane];
+        if (chunk == 0 && lane < ib - k) top[k * CTA_NB + k + lane] = rest[lane];
         if (pos == (int)gpos) {
             live = false;                                // the pivot row is U row k
             pos = k;
@@ -167,13 +171,13 @@ __device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, 
         T l = a[0] * r;
         if (recip_special(piv)) l = nz ? rscale(a[0], piv, recip(piv)) : a[0];
         if (row) sP[k * ldp + i] = l;                    // (rows already chosen: never read)
-        if (k + 1 < ib) cta_step<T>(a, l, rest, s, buf ^ 1, chunk, live, pos, k + 1, ib - k);
+        if (k + 1 < ib) cta_step(a, l, rest, s, buf ^ 1, chunk, live, pos, k + 1, ib - k);
     }
     // pivoted order: every row to its position, in shared memory and in A.  A row's
     // L entries are its own stores (no barrier needed to read them back); a top row
     // goes on with its U entries.
     const int nl = pos < ib ? pos : ib;
-    if (row) {
+    if (row && MLU_BC2(pos, 0, pm, 1, 701)) {
 #pragma unroll
         for (int j = 0; j < CTA_NB; j++)
             if (j < nl) a[j] = sP[j * ldp + i];
@@ -181,11 +185,11 @@ __device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, 
         if (i < ib) s.dst[i] = pos >= ib ? pos : -1;
     }
     __syncthreads();
-    if (row) {
+    if (row && MLU_BC2(pos, 0, pm, 1, 704)) {
 #pragma unroll
         for (int j = 0; j < CTA_NB; j++)
             if (j < ib) {
-                const T v = j < nl ? a[j] : s.top[pos][j];
+                const T v = j < nl ? a[j] : top[pos * CTA_NB + j];
                 sP[j * ldp + pos] = v;
                 Ap[pos + (size_t)j * lda] = v;
             }
@@ -217,16 +221,16 @@ __device__ __forceinline__ void cta_lds(float (&v)[2], const float *p)
     v[0] = x.x, v[1] = x.y;
 }
 
-// The panel's interchanges on column `col` (pointer to its row j0), and with
+// The panel's interchanges on column `col` (pointer to its row j0, pm rows), and with
 // SOLVE U12 = L11^{-1} A12 for it, also stored to sU (stride ldu).  FULL: ib is CTA_NB.
-template <typename T, bool SOLVE, bool FULL>
-__device__ __forceinline__ void cta_column(T *col, int ib, const T *sP, int ldp, const CtaPanel<T> &s, T *sU, int ldu)
+template <bool SOLVE, bool FULL, typename T, int NCH>
+__device__ __forceinline__ void cta_column(T *col, int pm, int ib, const T *sP, int ldp, const CtaPanel<T, NCH> &s, T *sU, int ldu)
 {
     T v[CTA_NB];
     const volatile int *slot = s.slot, *dst = s.dst;     // re-read: registers are short here
 #pragma unroll
     for (int q = 0; q < CTA_NB; q++)
-        if (FULL || q < ib) v[q] = col[slot[q]];
+        if (FULL || q < ib) v[q] = MLU_BC2(slot[q], 0, pm, 1, 702) ? col[slot[q]] : T(0);
 #pragma unroll
     for (int q0 = 0; q0 < CTA_NB; q0 += 4) {             // the rows the pivots left
         T w[4];
@@ -235,7 +239,7 @@ __device__ __forceinline__ void cta_column(T *col, int ib, const T *sP, int ldp,
             if ((FULL || q0 + q < ib) && dst[q0 + q] >= 0) w[q] = col[q0 + q];
 #pragma unroll
         for (int q = 0; q < 4; q++)
-            if ((FULL || q0 + q < ib) && dst[q0 + q] >= 0) col[dst[q0 + q]] = w[q];
+            if ((FULL || q0 + q < ib) && dst[q0 + q] >= 0 && MLU_BC2(dst[q0 + q], 0, pm, 1, 703)) col[dst[q0 + q]] = w[q];
     }
     if (SOLVE) {
 #pragma unroll
@@ -303,13 +307,13 @@ __device__ __forceinline__ int cta_rot(int k) { return (int)((unsigned)k * 0x9E3
 
 // The factorisation of the m x n matrix at A (m, n <= blockDim.x), and the
 // interchanges applied to its nrhs right-hand sides.  smem: cta_lu_smem bytes for
-// the row strides ldp >= cta_ld(m), ldu >= cta_ld(n).  nb: panel width, 8 or 16;
+// the row strides ldp >= cta_ldp(m), ldu >= cta_ldu(n, nb).  nb: panel width, 8 or 16;
 // small: 2 x 2 elements per thread in every update.  `rot` turns the assignment of rows and columns to warps, so that the short panels and steps
 // of different matrices do not all load the same scheduler (cta_rot).  Sets *info_out to the
 // first zero pivot (1-based) or 0; ends with a barrier.
-template <typename T>
+template <typename T, int NCH>
 __device__ __forceinline__ void cta_lu(int m, int n, T *A, int lda, int *ipiv, int nrhs, T *B, int ldb,
-                                      unsigned char *smem, int ldp, int ldu, CtaPanel<T> &s, int nb, bool small, int rot, int *info_out)
+                                      unsigned char *smem, int ldp, int ldu, CtaPanel<T, NCH> &s, int nb, bool small, int rot, int *info_out)
 {
     T *sP = reinterpret_cast<T *>(smem), *sU = sP + CTA_NB * ldp;
     const int tid = threadIdx.x, nt = blockDim.x, mn = min(m, n);
@@ -317,7 +321,7 @@ __device__ __forceinline__ void cta_lu(int m, int n, T *A, int lda, int *ipiv, i
         const int ib = min(nb, mn - j0);
         T *Ap = A + j0 + (size_t)j0 * lda;
         const int vtid = (tid + 32 * (step & 7)) & (nt - 1);   // nt is a power of two
-        const int il = cta_panel<T>(m - j0, ib, Ap, lda, sP, ldp, s, vtid);
+        const int il = cta_panel<T>(m - j0, ib, Ap, lda, sP, ldp, sU, s, vtid);
         // every thread with a row knows il: the one with row 0 keeps the first
         if (vtid == 0) {
             if (step == rot) *info_out = il;             // (the panel's barriers order these writes)
@@ -329,11 +333,11 @@ __device__ __forceinline__ void cta_lu(int m, int n, T *A, int lda, int *ipiv, i
         for (int c = vtid; c < rn + nrhs + j0; c += nt) {
             if (c < rn) {
                 T *col = Ap + (size_t)(ib + c) * lda;
-                if (ib == CTA_NB) cta_column<T, true, true>(col, ib, sP, ldp, s, sU + c, ldu);
-                else cta_column<T, true, false>(col, ib, sP, ldp, s, sU + c, ldu);
+                if (ib == CTA_NB) cta_column<true, true>(col, m - j0, ib, sP, ldp, s, sU + c, ldu);
+                else cta_column<true, false>(col, m - j0, ib, sP, ldp, s, sU + c, ldu);
             } else {
                 T *col = c < rn + nrhs ? B + j0 + (size_t)(c - rn) * ldb : A + j0 + (size_t)(c - rn - nrhs) * lda;
-                cta_column<T, false, false>(col, ib, sP, ldp, s, nullptr, 0);
+                cta_column<false, false>(col, m - j0, ib, sP, ldp, s, (T *)nullptr, 0);
             }
         }
         __syncthreads();

@@ -114,7 +114,7 @@ vb_lu_kernel(const int *m_arr, const int *n_arr, const int *nrhs_arr, T **dA_arr
              VbTune tune)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ __align__(16) CtaPanel<T> s_panel;
+    __shared__ __align__(16) CtaPanel<T, CTA_MAX_N / 32> s_panel;
     __shared__ int s_item;
     const int tid = threadIdx.x;
     // the solve's diagonal block, then its right-hand sides, in the same memory
@@ -192,7 +192,7 @@ __global__ void vb_check_kernel(const int *m, const int *n, const int *nrhs, con
 template <typename T>
 size_t vb_smem_bytes(int max_m, int max_n, int max_nrhs)
 {
-    size_t need = cta_lu_smem<T>(max(max_m, 1), max(max_n, 1));
+    size_t need = cta_lu_smem<T>(max(max_m, 1), max(max_n, 1), 0);
     if (max_nrhs > 0) need = max(need, sizeof(Diag<T>) + (size_t)VB_NR * solve_ldx<T>(max_n) * sizeof(T));
     return need;
 }
@@ -249,7 +249,7 @@ magma_int_t vb_run(const int *m, const int *n, const int *nrhs, int max_m, int m
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vb_lu_kernel<T>, VB_THREADS, smem);
     const int grid = max(1, min(batch, sms * max(per_sm, 1)));
     MLU_LAUNCH(mlu::KC_VB_LU, q->stream, vb_lu_kernel<T><<<grid, VB_THREADS, smem, q->stream>>>(m, n, nrhs, dA, ldda, ipiv, dB, lddb, info,
-                                                          order, counter, batch, cta_ld(max(max_m, 1)), cta_ld(max(max_n, 1)), tune));
+                                                          order, counter, batch, cta_ldp(max(max_m, 1)), cta_ldu(max(max_n, 1), 0), tune));
     MLU_CHECK_LAUNCH();
     return 0;
 }
