@@ -155,7 +155,8 @@ magma_int_t chol_factor(int n, T **dA, int lda, int *info, int batch, magma_queu
 
 constexpr int CHOL_NR = 4;
 
-template <typename T>
+// One CTA per (matrix, group of NR right-hand sides).
+template <typename T, int NR>
 __global__ void __launch_bounds__(256)
 chol_solve_kernel(int n, int nrhs, T **dA_array, int lda, T **dB_array, int ldb)
 {
@@ -163,33 +164,49 @@ chol_solve_kernel(int n, int nrhs, T **dA_array, int lda, T **dB_array, int ldb)
     __shared__ __align__(16) Diag<T> sD;
     T *sB = reinterpret_cast<T *>(smem_raw);
     const int mat = blockIdx.y, tid = threadIdx.x, ldx = solve_ldx<T>(n);
-    const int c0 = blockIdx.x * CHOL_NR, nr = min(CHOL_NR, nrhs - c0);
+    const int c0 = blockIdx.x * NR, nr = min(NR, nrhs - c0);
     T *B = dB_array[mat] + (size_t)c0 * ldb;
-    for (int e = tid; e < CHOL_NR * n; e += blockDim.x) {
+    for (int e = tid; e < NR * n; e += blockDim.x) {
         const int c = e / n, i = e % n;
         sB[c * ldx + i] = c < nr ? B[i + (size_t)c * ldb] : T(0);
     }
-    chol_solve_smem<T, solve_cg<T, CHOL_NR>()>(n, dA_array[mat], lda, sB, ldx, nr, sD);
+    chol_solve_smem<T, solve_cg<T, NR>()>(n, dA_array[mat], lda, sB, ldx, nr, sD);
     for (int e = tid; e < nr * n; e += blockDim.x) {
         const int c = e / n, i = e % n;
         B[i + (size_t)c * ldb] = sB[c * ldx + i];
     }
 }
 
+template <typename T, int NR>
+static size_t chol_solve_dyn_max()
+{
+    static size_t dyn_cache[MLU_MAX_DEVICES];
+    return mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(chol_solve_kernel<T, NR>); });
+}
+
+template <typename T, int NR>
+static void launch_chol_solve(int n, int nrhs, T **dA, int lda, T **dB, int ldb, int batch, cudaStream_t s)
+{
+    const int threads = min(256, max(64, (n + 31) / 32 * 32));
+    MLU_LAUNCH(mlu::KC_GETRS, s,
+               chol_solve_kernel<T, NR><<<dim3((nrhs + NR - 1) / NR, batch), threads,
+                                          (size_t)NR * solve_ldx<T>(n) * sizeof(T), s>>>(n, nrhs, dA, lda, dB, ldb));
+}
+
 template <typename T>
 magma_int_t chol_solve(int n, int nrhs, T **dA, int lda, T **dB, int ldb, int batch,
                        magma_queue_t q)
 {
-    const size_t smem = (size_t)CHOL_NR * solve_ldx<T>(n) * sizeof(T);
-    static size_t dyn_cache[MLU_MAX_DEVICES];
-    const size_t dyn_max = mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(chol_solve_kernel<T>); });
-    if (smem > dyn_max) return MAGMA_ERR_NOT_SUPPORTED;
-    const int threads = min(256, max(64, (n + 31) / 32 * 32));
+    // Four columns beside a 32 x 33 block set the largest order; where the padded columns
+    // and the larger block of the sweeps do not fit, a CTA takes one column.
+    const size_t dm = chol_solve_dyn_max<T, CHOL_NR>(), block = 32 * 33 * sizeof(T);
+    if ((size_t)CHOL_NR * n * sizeof(T) + block > dm + sizeof(Diag<T>)) return MAGMA_ERR_NOT_SUPPORTED;
+    const bool one = (size_t)CHOL_NR * solve_ldx<T>(n) * sizeof(T) > dm;
+    if (one) chol_solve_dyn_max<T, 1>();
     for (int b0 = 0; b0 < batch; b0 += MLU_MAX_GRID_Y) {
         const int nb = min(batch - b0, (int)MLU_MAX_GRID_Y);
-        MLU_LAUNCH(mlu::KC_GETRS, q->stream,
-                   chol_solve_kernel<T><<<dim3((nrhs + CHOL_NR - 1) / CHOL_NR, nb), threads, smem, q->stream>>>(
-                       n, nrhs, dA + b0, lda, dB + b0, ldb));
+        if (one) launch_chol_solve<T, 1>(n, nrhs, dA + b0, lda, dB + b0, ldb, nb, q->stream);
+        else launch_chol_solve<T, CHOL_NR>(n, nrhs, dA + b0, lda, dB + b0, ldb, nb, q->stream);
     }
     MLU_CHECK_LAUNCH();
     return 0;

@@ -552,6 +552,7 @@ constexpr float GM_INNER_TOL = 1e-4f;
 constexpr int GM_THREADS = 256;
 constexpr int GM_WARPS = GM_THREADS / 32;
 constexpr int GM_NRHS_MAX = 8;
+constexpr int GM_N_MAX = 2200;      // the right-hand sides and the Hessenberg matrices in shared memory
 // A refinement step whose residual 2-norm did not at least halve (any
 // right-hand side) ends the refinement of that matrix: it is marked as not
 // converged and goes to the FP64 re-solve (the reference instead runs all its
@@ -597,11 +598,19 @@ __device__ __forceinline__ void gm_block_sum(F (&v)[NR], F (*red)[NR], F *out)
     __syncthreads();
 }
 
+// The Arnoldi vectors of one step; the solves' diagonal block lies in their place, which
+// holds nothing while a solve runs.
+template <int NR>
+__host__ __device__ constexpr int gm_w_floats(int n)
+{
+    const int d = (int)(sizeof(Diag<float>) / sizeof(float));
+    return NR * n > d ? NR * n : d;
+}
 template <int NR>
 __host__ __device__ inline size_t gm_smem_bytes(int n)
 {
     const int m = n < GM_INNER_MAX ? n : GM_INNER_MAX;
-    return sizeof(float) * ((size_t)NR * (solve_ldx<float>(n) + n) + (size_t)NR * (m + 1) * m + (size_t)NR * (3 * m + 1));
+    return sizeof(float) * ((size_t)NR * solve_ldx<float>(n) + gm_w_floats<NR>(n) + (size_t)NR * (m + 1) * m + (size_t)NR * (3 * m + 1));
 }
 
 // check (as ir_solve_kernel) + GMRES correction X += d for the nrhs <= NR
@@ -617,7 +626,6 @@ gm_correction_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, c
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ float s_red[GM_WARPS][NR], s_sum[NR];
     __shared__ double s_red64[GM_WARPS][NR], s_sum64[NR];
-    __shared__ __align__(16) Diag<float> sD;
     __shared__ int s_go, s_act[NR], s_k[NR], s_any;
     const int mat = blockIdx.y, tid = threadIdx.x;
     const int n = sh.N(mat), nrhs = sh.NR(mat), lddx = sh.LDX(mat);
@@ -625,8 +633,9 @@ gm_correction_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, c
     const int m = min(GM_INNER_MAX, n);
     const int ldx = solve_ldx<float>(n);
     float *sB = reinterpret_cast<float *>(smem_raw);   // [NR][ldx]: preconditioner input / output
-    float *sW = sB + NR * ldx;                           // [NR][n]: Arnoldi vector
-    float *sH = sW + NR * n;                           // [NR][m+1][m]: Hessenberg matrices
+    float *sW = sB + NR * ldx;                         // [NR][n]: Arnoldi vector
+    Diag<float> &sD = *reinterpret_cast<Diag<float> *>(sW);   // ... or the solve's diagonal block
+    float *sH = sW + gm_w_floats<NR>(n);               // [NR][m+1][m]: Hessenberg matrices
     float *sCs = sH + NR * (m + 1) * m;                // [NR][m]
     float *sSn = sCs + NR * m;                         // [NR][m]
     float *sRs = sSn + NR * m;                         // [NR][m+1]: rotated right-hand side, then y
@@ -1167,7 +1176,7 @@ ir_run(int prec, const IrShape &sh, double **dA_array, magma_int_t **dipiv_array
     if (n == 0 || nrhs == 0 || batchCount <= 0) return 0;
     // shared-memory limits of the correction solve and the residual kernels
     if (!ir_fits("magma_dxgesv_batched", n, nrhs)) return MAGMA_ERR_NOT_SUPPORTED;
-    if (gm && (vb || nrhs > GM_NRHS_MAX || gm_smem_bytes<GM_NRHS_MAX>(n) > gm_dyn_max()))
+    if (gm && (vb || nrhs > GM_NRHS_MAX || n > GM_N_MAX || gm_smem_bytes<GM_NRHS_MAX>(n) > gm_dyn_max()))
         return MAGMA_ERR_NOT_SUPPORTED;
 
     cudaStream_t s = queue->stream;

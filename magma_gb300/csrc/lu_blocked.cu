@@ -1022,8 +1022,11 @@ magma_int_t blocked_getrs(bool trans, int n, int nrhs, T **dA, int ldda, int **i
     if (batch <= 0 || n == 0 || nrhs == 0) return MAGMA_SUCCESS;
     static size_t dyn_cache[MLU_MAX_DEVICES];
     const size_t dm = mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(getrs_kernel<T, false, 1>); });
-    // the largest order: four (or, with more right-hand sides, eight) columns in shared memory
-    if ((size_t)(nrhs <= 4 ? 4 : SOLVE_NC) * n * sizeof(T) > dm) return MAGMA_ERR_NOT_SUPPORTED;
+    // the largest order: four (or, with more right-hand sides, eight) columns in shared
+    // memory beside a 32 x 33 block (the sweeps' own is larger, and their columns are
+    // padded: near that order fewer columns go to a CTA, below)
+    if ((size_t)(nrhs <= 4 ? 4 : SOLVE_NC) * n * sizeof(T) + 32 * 33 * sizeof(T) > dm + sizeof(Diag<T>))
+        return MAGMA_ERR_NOT_SUPPORTED;
     // Right-hand sides per CTA: eight, fewer while that leaves SMs without a CTA
     // (the sweeps of different right-hand sides do not wait for one another) or
     // while they do not fit.  FP32: as many as one update task takes.
