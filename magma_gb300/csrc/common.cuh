@@ -23,6 +23,12 @@ struct magma_queue {
     // scratch space (never by the factor/solve routines themselves).
     void *work;
     size_t work_bytes;
+    // What a refinement on this queue shows the host while it runs (ir.cu): a page-locked
+    // word and the event after which it is written, made at the first use, freed with the
+    // queue, and used by one call at a time (look_busy, taken atomically).
+    int *look;
+    cudaEvent_t look_event;
+    int look_busy;
 };
 
 namespace mlu {

@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "trace.cuh"
 #include "convert.cuh"
+#include "ir_loop.cuh"
 #include "solve_core.cuh"
 #include "chol_core.cuh"
 
@@ -842,7 +843,9 @@ gm_correction_kernel(IrShape sh, float **dAs_array, int ldas, const int *perm, c
     }
 }
 
-__global__ void ir_final_kernel(IrShape sh, unsigned long long *stats, int *iter, int itermax,
+// The verdict on the matrices still active after `done` of at most itermax iterations
+// (residual `done` is the last one formed).
+__global__ void ir_final_kernel(IrShape sh, unsigned long long *stats, int *iter, int itermax, int done,
                                 double tol, int batch, int *failed_count,
                                 const int *inner_total = nullptr)
 {
@@ -850,9 +853,9 @@ __global__ void ir_final_kernel(IrShape sh, unsigned long long *stats, int *iter
     if (mat >= batch) return;
     unsigned long long *st = stats + (size_t)mat * IR_STATS_WORDS;
     if (st[1] == IR_ACTIVE) {
-        if (ir_converged(st, itermax & 1, sh.N(mat), sh.NR(mat), tol)) {
+        if (ir_converged(st, done & 1, sh.N(mat), sh.NR(mat), tol)) {
             st[1] = IR_CONVERGED;
-            iter[mat] = inner_total ? inner_total[mat] : itermax;
+            iter[mat] = inner_total ? inner_total[mat] : done;
         } else {
             st[1] = IR_FAILED;
             iter[mat] = -itermax - 1;
@@ -1124,31 +1127,74 @@ static size_t solve_dyn_max()
 
 using namespace mlu;
 
-// The refinement iterations: correct(it) tests convergence and corrects, resid(it)
-// forms the residual of parity it & 1.  With `poll` (the call waits for the device
-// at its end anyway) the host looks after every second iteration whether any matrix
-// is still being refined, and leaves the loop when none is: an iteration without
-// work is two launches of about 2.3 us, and thirty of them were most of a call on a
-// small batch (SPD refinement of 256 matrices of order 256: 1196 -> 876 us, pointer arrays in one launch included).  A
-// look costs about 15 us of idle device, so it is not taken after every iteration.
-template <typename C, typename R>
-static magma_int_t ir_iterate(const IrShape &sh, const unsigned long long *stats, int itermax, double tol, int batch,
-                              int *active, bool poll, cudaStream_t s, C correct, R resid)
-{
-    for (int it = 0; it < itermax; it++) {
-        correct(it);
-        resid(it + 1);
-        if (!poll || (it & 1) == 0 || it + 1 >= itermax) continue;
-        int left = 0;
-        MLU_LAUNCH(mlu::KC_OTHER, s, ir_active_kernel<<<1, 1024, 0, s>>>(sh, stats, (it + 1) & 1, tol, batch, active));
-        cudaMemcpyAsync(&left, active, sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess) return MAGMA_ERR_UNKNOWN;
-        if (left == 0) {
-            correct(it + 1);                     // marks them converged
-            break;
+// How many matrices are still being refined, as the host loop asks for it (ir_loop.cuh).
+// The kernel writes the number into a page-locked word of the queue, made at the queue's
+// first refinement; while another thread's call uses that word, or where there is none,
+// into `active` (device memory of this call), and wait() copies it.
+struct ActiveLook {
+    const IrShape &sh;
+    const unsigned long long *stats;
+    double tol;
+    int batch, *active;
+    magma_queue_t q;
+    bool word;
+
+    ActiveLook(const IrShape &sh_, const unsigned long long *stats_, double tol_, int batch_, int *active_, magma_queue_t q_)
+        : sh(sh_), stats(stats_), tol(tol_), batch(batch_), active(active_), q(q_), word(false)
+    {
+        if (__atomic_exchange_n(&q->look_busy, 1, __ATOMIC_ACQUIRE) != 0) return;
+        if (q->look == nullptr) {
+            // (not an operation that another thread's capture has to see)
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            void *p = nullptr;
+            if (cudaEventCreateWithFlags(&q->look_event, cudaEventDisableTiming) != cudaSuccess) q->look_event = nullptr;
+            else if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) q->look = (int *)p;
+            else cudaEventDestroy(q->look_event);
+            if (q->look == nullptr) cudaGetLastError();
+            cudaThreadExchangeStreamCaptureMode(&mode);
         }
+        word = q->look != nullptr;
+        if (!word) __atomic_store_n(&q->look_busy, 0, __ATOMIC_RELEASE);
     }
-    return 0;
+    ~ActiveLook()
+    {
+        if (word) __atomic_store_n(&q->look_busy, 0, __ATOMIC_RELEASE);
+    }
+    ActiveLook(const ActiveLook &) = delete;
+
+    int post(int it)
+    {
+        int *to = active;
+        if (word && cudaHostGetDevicePointer((void **)&to, q->look, 0) != cudaSuccess) return MAGMA_ERR_UNKNOWN;
+        MLU_LAUNCH(mlu::KC_OTHER, q->stream, ir_active_kernel<<<1, 1024, 0, q->stream>>>(sh, stats, it & 1, tol, batch, to));
+        if (cudaGetLastError() != cudaSuccess) return MAGMA_ERR_UNKNOWN;
+        if (word && cudaEventRecord(q->look_event, q->stream) != cudaSuccess) return MAGMA_ERR_UNKNOWN;
+        return 0;
+    }
+    int wait(int *left)
+    {
+        if (word) {
+            if (cudaEventSynchronize(q->look_event) != cudaSuccess) return MAGMA_ERR_UNKNOWN;
+            *left = *(volatile int *)q->look;
+            return 0;
+        }
+        if (cudaMemcpyAsync(left, active, sizeof(int), cudaMemcpyDeviceToHost, q->stream) != cudaSuccess ||
+            cudaStreamSynchronize(q->stream) != cudaSuccess)
+            return MAGMA_ERR_UNKNOWN;
+        return 0;
+    }
+};
+
+// ir_iterate; the host looks at the number of active matrices when the call waits for
+// the device at its end anyway (`poll`).
+template <typename C, typename R>
+static magma_int_t ir_loop(const IrShape &sh, const unsigned long long *stats, int itermax, double tol, int batch,
+                           int *active, bool poll, magma_queue_t q, C correct, R resid, int *done)
+{
+    if (!poll) return ir_iterate(itermax, (ActiveLook *)nullptr, correct, resid, done);
+    ActiveLook look(sh, stats, tol, batch, active, q);
+    return ir_iterate(itermax, &look, correct, resid, done);
 }
 
 // The refinement driver for factorisation precision `prec`: 900 FP32
@@ -1245,12 +1291,13 @@ ir_run(int prec, const IrShape &sh, double **dA_array, magma_int_t **dipiv_array
     };
     solve(-1);
     residual<false>(sh, dA_array, dB_array, dX_array, R, stats, 0, batchCount, s);
-    rc = ir_iterate(
-        sh, stats, itermax, tol, batchCount, count + 3, fallback != 0, s, [&](int it) { gm ? gmres(it) : solve(it); },
-        [&](int it) { residual<false>(sh, dA_array, dB_array, dX_array, R, stats, it & 1, batchCount, s); });
+    int done = 0;
+    rc = ir_loop(
+        sh, stats, itermax, tol, batchCount, count + 3, fallback != 0, queue, [&](int it) { gm ? gmres(it) : solve(it); },
+        [&](int it) { residual<false>(sh, dA_array, dB_array, dX_array, R, stats, it & 1, batchCount, s); }, &done);
     if (rc != 0) return rc;
     MLU_LAUNCH(mlu::KC_OTHER, s, ir_final_kernel<<<mlu_ceildiv(batchCount, 256), 256, 0, s>>>(
-        sh, stats, diter_array, itermax, tol, batchCount, count, inner));
+        sh, stats, diter_array, itermax, done, tol, batchCount, count, inner));
     MLU_CHECK_LAUNCH();
     if (!fallback) return 0;
 
@@ -1376,14 +1423,13 @@ ir_run_adjoint(const IrShape &sh, double **dA_array, magma_int_t **dipiv_array, 
     };
     solve(-1);
     residual<true>(sh, dA_array, dG_array, dGB_array, R, stats, 0, batchCount, s);
-    {
-        const magma_int_t rc = ir_iterate(
-            sh, stats, itermax, tol, batchCount, count + 3, fallback != 0, s, solve,
-            [&](int it) { residual<true>(sh, dA_array, dG_array, dGB_array, R, stats, it & 1, batchCount, s); });
-        if (rc != 0) return rc;
-    }
+    int done = 0;
+    const magma_int_t rl = ir_loop(
+        sh, stats, itermax, tol, batchCount, count + 3, fallback != 0, queue, solve,
+        [&](int it) { residual<true>(sh, dA_array, dG_array, dGB_array, R, stats, it & 1, batchCount, s); }, &done);
+    if (rl != 0) return rl;
     MLU_LAUNCH(mlu::KC_OTHER, s, ir_final_kernel<<<mlu_ceildiv(batchCount, 256), 256, 0, s>>>(
-        sh, stats, diter_array, itermax, tol, batchCount, count));
+        sh, stats, diter_array, itermax, done, tol, batchCount, count));
     MLU_CHECK_LAUNCH();
 
     // FP64 transposed solves for matrices the refinement did not solve (without

@@ -85,6 +85,10 @@ extern "C" void magma_queue_destroy_internal(magma_queue_t queue, const char *, 
     if (!queue) return;
     if (queue->stream) cudaStreamSynchronize(queue->stream);
     if (queue->work) cudaFree(queue->work);
+    if (queue->look) {
+        cudaEventDestroy(queue->look_event);
+        cudaFreeHost(queue->look);
+    }
     if (queue->own_stream) cudaStreamDestroy(queue->stream);
     free(queue);
 }
