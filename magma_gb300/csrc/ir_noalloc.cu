@@ -101,7 +101,12 @@ magma_dsgesv_batched_noalloc(magma_int_t n, magma_int_t nrhs, double **dA_array,
     void *scratch = scratch_address(queue->device);
     if (!scratch) return MAGMA_ERR_UNKNOWN;
     size_t have = NOALLOC_SCRATCH_BYTES;
-    return magma_dsgesv_batched_work(n, nrhs, dA_array, ldda, dipiv_array, dB_array, lddb,
-                                     dX_array, lddx, dinfo_array, diter_array, 30, 0.0, 1,
-                                     scratch, &have, batchCount, queue);
+    // No page-locked word for the queue either: while it is taken, the refinement makes
+    // none and reads its count of active matrices from the scratch.
+    const int taken = __atomic_exchange_n(&queue->look_busy, 1, __ATOMIC_ACQUIRE);
+    rc = magma_dsgesv_batched_work(n, nrhs, dA_array, ldda, dipiv_array, dB_array, lddb,
+                                   dX_array, lddx, dinfo_array, diter_array, 30, 0.0, 1,
+                                   scratch, &have, batchCount, queue);
+    if (!taken) __atomic_store_n(&queue->look_busy, 0, __ATOMIC_RELEASE);
+    return rc;
 }
