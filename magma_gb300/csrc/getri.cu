@@ -37,11 +37,7 @@ getri_kernel(int n, T **dA_array, int ldda, int **ipiv_array, T **dInv_array, in
         const int c = e / n, i = e % n;
         sB[c * ldx + i] = (c < nr && i == j0 + c) ? T(1) : T(0);
     }
-    if (tid < nr) {
-        int tau[1] = {j0 + tid};
-        resolve_rows(tau, ipiv, n);
-        s_col[tid] = tau[0];
-    }
+    if (tid < nr) s_col[tid] = resolve_row(j0 + tid, ipiv, n);
     solve_smem<T, false, solve_cg<T, GETRI_NR>()>(n, dA_array[mat], ldda, sB, ldx, nr, sD);
     T *Inv = dInv_array[mat];
     for (int e = tid; e < nr * n; e += blockDim.x) {

@@ -983,36 +983,33 @@ constexpr int SOLVE_THREADS = 256;
 constexpr int SOLVE_NC = 8;                // right-hand sides per CTA, at most
 
 // CG: right-hand sides per update task (FP32: nc is a multiple of it).
-// `stage_piv`: the pivots fit in shared memory behind the right-hand sides.
 template <typename T, bool TRANS, int CG>
 __global__ void __launch_bounds__(SOLVE_THREADS, sizeof(T) == 8 ? 2 : 3)
-getrs_kernel(int n, int nrhs, T **dA_array, int ldda, int **ipiv_array, T **dB_array, int lddb, int nc,
-             int stage_piv)
+getrs_kernel(int n, int nrhs, T **dA_array, int ldda, int **ipiv_array, T **dB_array, int lddb, int nc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(16) Diag<T> sD;
     T *sB = reinterpret_cast<T *>(smem_raw);   // [nc][ldx]
     const int ldx = solve_ldx<T>(n);
-    int *s_piv = stage_piv ? reinterpret_cast<int *>(sB + (size_t)nc * ldx) : nullptr;
     const int mat = blockIdx.y;
     const int c0 = blockIdx.x * nc;
     const int nr = min(nc, nrhs - c0);
     const T *A = dA_array[mat];
     const int *ipiv = ipiv_array ? ipiv_array[mat] : nullptr;   // null: no interchanges
     T *B = dB_array[mat] + (size_t)c0 * lddb;
-    move_rhs<T, false>(n, TRANS ? nullptr : ipiv, s_piv, B, lddb, sB, ldx, nr, nc);
+    move_rhs<T, false>(n, TRANS ? nullptr : ipiv, B, lddb, sB, ldx, nr, nc);
     solve_smem<T, TRANS, CG>(n, A, ldda, sB, ldx, nr, sD);
-    move_rhs<T, true>(n, TRANS ? ipiv : nullptr, s_piv, B, lddb, sB, ldx, nr, nc);
+    move_rhs<T, true>(n, TRANS ? ipiv : nullptr, B, lddb, sB, ldx, nr, nc);
 }
 
 template <typename T, bool TRANS, int CG>
 static void launch_getrs(dim3 grid, int threads, size_t smem, cudaStream_t s, int n, int nrhs, T **A, int ldda,
-                         int **P, T **B, int lddb, int nc, int stage_piv)
+                         int **P, T **B, int lddb, int nc)
 {
     static size_t dyn_cache[MLU_MAX_DEVICES];
     mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(getrs_kernel<T, TRANS, CG>); });
     MLU_LAUNCH(mlu::KC_GETRS, s, getrs_kernel<T, TRANS, CG><<<grid, threads, smem, s>>>(
-        n, nrhs, A, ldda, P, B, lddb, nc, stage_piv));
+        n, nrhs, A, ldda, P, B, lddb, nc));
 }
 
 template <typename T>
@@ -1034,8 +1031,7 @@ magma_int_t blocked_getrs(bool trans, int n, int nrhs, T **dA, int ldda, int **i
     int nc = sizeof(T) == 4 ? (nrhs == 1 ? 1 : nrhs <= 4 ? 4 : SOLVE_NC) : min(nrhs, SOLVE_NC);
     while (nc > 1 && ((long long)batch * mlu_ceildiv(nrhs, nc) < mlu_sm_count() || nc * col > dm))
         nc = sizeof(T) == 4 ? (nc == 8 ? 4 : 1) : (nc + 1) / 2;
-    const bool stage_piv = ipiv != nullptr && nc * col + (size_t)n * sizeof(int) <= dm;
-    const size_t smem = nc * col + (stage_piv ? (size_t)n * sizeof(int) : 0);
+    const size_t smem = nc * col;
     // FP64: four warps use the whole FP64 pipe, eight when an SM has one CTA; FP32:
     // one thread per row up to 256
     const int threads = sizeof(T) == 8 ? ((long long)batch * mlu_ceildiv(nrhs, nc) >= 2 * mlu_sm_count() ? 128 : 256)
@@ -1048,8 +1044,8 @@ magma_int_t blocked_getrs(bool trans, int n, int nrhs, T **dA, int ldda, int **i
         int **P = ipiv ? ipiv + b0 : nullptr;
         auto go = [&](auto cg) {
             constexpr int CG = decltype(cg)::value;
-            if (trans) launch_getrs<T, true, CG>(grid, threads, smem, s, n, nrhs, A, ldda, P, B, lddb, nc, stage_piv);
-            else launch_getrs<T, false, CG>(grid, threads, smem, s, n, nrhs, A, ldda, P, B, lddb, nc, stage_piv);
+            if (trans) launch_getrs<T, true, CG>(grid, threads, smem, s, n, nrhs, A, ldda, P, B, lddb, nc);
+            else launch_getrs<T, false, CG>(grid, threads, smem, s, n, nrhs, A, ldda, P, B, lddb, nc);
         };
         if (nc == 1) go(std::integral_constant<int, 1>{});
         else if constexpr (sizeof(T) == 8) go(std::integral_constant<int, 2>{});

@@ -141,9 +141,9 @@ vb_lu_kernel(const int *m_arr, const int *n_arr, const int *nrhs_arr, T **dA_arr
                 const int nr = min(VB_NR, nrhs - c0);
                 T *Bc = B + (size_t)c0 * ldb;
                 __syncthreads();
-                move_rhs<T, false>(n, nullptr, nullptr, Bc, ldb, sT, ldx, nr, VB_NR);
+                move_rhs<T, false>(n, nullptr, Bc, ldb, sT, ldx, nr, VB_NR);
                 solve_smem<T, false, solve_cg<T, VB_NR>(), 16>(n, A, lda, sT, ldx, nr, sD);
-                move_rhs<T, true>(n, nullptr, nullptr, Bc, ldb, sT, ldx, nr, VB_NR);
+                move_rhs<T, true>(n, nullptr, Bc, ldb, sT, ldx, nr, VB_NR);
             }
         }
     }
@@ -163,12 +163,11 @@ vb_getrs_kernel(const int *n_arr, const int *nrhs_arr, T **dA_array, const int *
     const int c0 = blockIdx.x * VB_SOLVE_NR;
     if (n <= 0 || c0 >= nrhs) return;
     const int nr = min(VB_SOLVE_NR, nrhs - c0), ldx = solve_ldx<T>(n);
-    int *s_piv = reinterpret_cast<int *>(sB + (size_t)VB_SOLVE_NR * ldx);
     const int ldb = lddb_arr[k];
     T *B = dB_array[k] + (size_t)c0 * ldb;
-    move_rhs<T, false>(n, TRANS ? nullptr : ipiv_array[k], s_piv, B, ldb, sB, ldx, nr, VB_SOLVE_NR);
+    move_rhs<T, false>(n, TRANS ? nullptr : ipiv_array[k], B, ldb, sB, ldx, nr, VB_SOLVE_NR);
     solve_smem<T, TRANS, solve_cg<T, VB_SOLVE_NR>()>(n, dA_array[k], ldda_arr[k], sB, ldx, nr, sD);
-    move_rhs<T, true>(n, TRANS ? ipiv_array[k] : nullptr, s_piv, B, ldb, sB, ldx, nr, VB_SOLVE_NR);
+    move_rhs<T, true>(n, TRANS ? ipiv_array[k] : nullptr, B, ldb, sB, ldx, nr, VB_SOLVE_NR);
 }
 
 // argument check + maxima, one small kernel: stats = {err_m, err_n, err_ldda, err_lddb,
@@ -268,7 +267,7 @@ magma_int_t vb_getrs_run(bool trans, const int *n, const int *nrhs, int max_n, i
 {
     if (batch <= 0 || max_n <= 0 || max_nrhs <= 0) return 0;
     if ((size_t)VB_NR * max_n * sizeof(T) > VB_SMEM_CAP) return MAGMA_ERR_NOT_SUPPORTED;
-    const size_t smem = (size_t)VB_SOLVE_NR * solve_ldx<T>(max_n) * sizeof(T) + (size_t)max_n * sizeof(int);
+    const size_t smem = (size_t)VB_SOLVE_NR * solve_ldx<T>(max_n) * sizeof(T);
     static size_t dyn_cache[2][MLU_MAX_DEVICES];
     const size_t dyn_max = trans ? mlu_device_cached(dyn_cache[1], [] { return mlu_allow_dynamic_smem(vb_getrs_kernel<T, true>); })
                                  : mlu_device_cached(dyn_cache[0], [] { return mlu_allow_dynamic_smem(vb_getrs_kernel<T, false>); });
