@@ -1032,10 +1032,13 @@ magma_int_t blocked_getrs(bool trans, int n, int nrhs, T **dA, int ldda, int **i
     while (nc > 1 && ((long long)batch * mlu_ceildiv(nrhs, nc) < mlu_sm_count() || nc * col > dm))
         nc = sizeof(T) == 4 ? (nc == 8 ? 4 : 1) : (nc + 1) / 2;
     const size_t smem = nc * col;
-    // FP64: four warps use the whole FP64 pipe, eight when an SM has one CTA; FP32:
-    // one thread per row up to 256
-    const int threads = sizeof(T) == 8 ? ((long long)batch * mlu_ceildiv(nrhs, nc) >= 2 * mlu_sm_count() ? 128 : 256)
-                                       : min(SOLVE_THREADS, max(64, (n + 31) / 32 * 32));
+    // FP64: four warps a CTA where an SM holds four CTAs, else eight, because fewer warps
+    // leave the pipe idle while coefficients are on their way (16 right-hand sides, N / T, us
+    // with four warps / eight: n = 400 b = 1000 5270 / 5530, 5980 / 6430; n = 600 b = 300
+    // 3150 / 3230, 3340 / 3530; n = 800 b = 300 8130 / 5480, 9450 / 6590; n = 1000 b = 300
+    // 13200 / 8830, 13700 / 9330).  FP32: one thread per row up to 256.
+    const bool four = (long long)batch * mlu_ceildiv(nrhs, nc) >= 2 * mlu_sm_count() && 4 * (smem + sizeof(Diag<T>)) <= dm;
+    const int threads = sizeof(T) == 8 ? (four ? 128 : 256) : min(SOLVE_THREADS, max(64, (n + 31) / 32 * 32));
     cudaStream_t s = q->stream;
     for (int b0 = 0; b0 < batch; b0 += MLU_MAX_GRID_Y) {
         const int nb = min(batch - b0, (int)MLU_MAX_GRID_Y);
