@@ -218,7 +218,8 @@ int oracle_max_threads(void)
  *   sgetrf(As) (info > 0: iter -3); X = 0, R = B;
  *   solve: X = X + (double)sgetrs(As, (float)R);
  *   residual: r_i = b_i, r_i = fma(-a_ij, x_j, r_i) for j ascending;
- *   norms: per column max|r|, max|x|; row sums over the columns (ascending);
+ *   norms: per column max|r|, max|x|; row sums over the columns (ascending); a
+ *   NaN among them makes its norm NaN, which meets no stopping rule;
  *   stop when every column has max|r_c| <= max|x_c| * anrm*eps*sqrt(n)
  *   (tol <= 0) or when rowmax|R| <= tol * (anrm * rowmax|X| * n * eps);
  *   checks after the initial solve (iter 0) and after each of itermax
@@ -418,8 +419,8 @@ static int dsgesv_impl(int n, int nrhs, double *A, int lda, const double *B, int
                 double rc = 0.0, xc = 0.0;
                 for (int i = 0; i < n; i++) {
                     double ra = fabs(R[i + (size_t)c * n]), xa = fabs(X[i + (size_t)c * ldx]);
-                    if (ra > rc) rc = ra;
-                    if (xa > xc) xc = xa;
+                    if (ra > rc || ra != ra) rc = ra;
+                    if (xa > xc || xa != xa) xc = xa;
                 }
                 if (!(rc <= xc * cte)) ok = 0;
             }
@@ -429,8 +430,8 @@ static int dsgesv_impl(int n, int nrhs, double *A, int lda, const double *B, int
                     rs += fabs(R[i + (size_t)c * n]);
                     xs += fabs(X[i + (size_t)c * ldx]);
                 }
-                if (rs > rrow) rrow = rs;
-                if (xs > xrow) xrow = xs;
+                if (rs > rrow || rs != rs) rrow = rs;
+                if (xs > xrow || xs != xs) xrow = xs;
             }
             if (tol > 0.0) ok = rrow <= tol * (anrm * xrow * (double)n * eps);
             if (ok) { state = 1; iter = gmres ? inner : it; break; }
@@ -548,8 +549,8 @@ int oracle_dsgesv_adjoint(int n, int nrhs, double *A, int lda, int *ipiv, const 
                     double rc = 0.0, xc = 0.0;
                     for (int i = 0; i < n; i++) {
                         double ra = fabs(R[i + (size_t)c * n]), xa = fabs(GB[i + (size_t)c * ldgb]);
-                        if (ra > rc) rc = ra;
-                        if (xa > xc) xc = xa;
+                        if (ra > rc || ra != ra) rc = ra;
+                        if (xa > xc || xa != xa) xc = xa;
                     }
                     if (!(rc <= xc * cte)) ok = 0;
                 }
@@ -559,8 +560,8 @@ int oracle_dsgesv_adjoint(int n, int nrhs, double *A, int lda, int *ipiv, const 
                         rs += fabs(R[i + (size_t)c * n]);
                         xs += fabs(GB[i + (size_t)c * ldgb]);
                     }
-                    if (rs > rrow) rrow = rs;
-                    if (xs > xrow) xrow = xs;
+                    if (rs > rrow || rs != rs) rrow = rs;
+                    if (xs > xrow || xs != xs) xrow = xs;
                 }
                 if (tol > 0.0) ok = rrow <= tol * (anrm * xrow * (double)n * eps);
                 if (ok) { state = 1; iter = it; break; }
