@@ -21,7 +21,7 @@ constexpr int GETRI_NR = 8;
 constexpr int GETRI_THREADS = 256;
 
 template <typename T>
-__global__ void __launch_bounds__(GETRI_THREADS)
+__global__ void __launch_bounds__(GETRI_THREADS, sizeof(T) == 8 ? 2 : 3)
 getri_kernel(int n, T **dA_array, int ldda, int **ipiv_array, T **dInv_array, int lddia)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
