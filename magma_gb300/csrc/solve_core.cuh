@@ -266,6 +266,7 @@ __device__ __forceinline__ void diag_cols(Diag<float> &D, float *x, int ldx, int
 #pragma unroll
     for (int s = 0; s < 2; s++) {
         const int o = 16 * ((s == 0) == ASC ? 0 : 1), o2 = 16 - o;   // this triangle's rows, the other's
+        if (o >= tb) continue;                   // a block of at most 16 rows: its second half is empty
         if (lane < nr) {
             float y[16];
 #pragma unroll
@@ -289,7 +290,7 @@ __device__ __forceinline__ void diag_cols(Diag<float> &D, float *x, int ldx, int
             for (int i = 0; i < 16; i++)
                 if (o + i < tb) xc[o + i] = y[i];
         }
-        if (s == 0) {
+        if (s == 0 && tb > 16) {
             __syncwarp();
             const int ts = min(16, tb - o);       // columns of the square (the rest are zero)
             for (int e = lane; e < 16 * nr; e += 32) {
