@@ -128,7 +128,7 @@ vb_lu_kernel(const int *m_arr, const int *n_arr, const int *nrhs_arr, T **dA_arr
         if (idx >= batch) break;
         const int k = order[idx];
         const int m = m_arr[k], n = n_arr[k], lda = ldda_arr[k];
-        const int nrhs = nrhs_arr ? nrhs_arr[k] : 0;
+        const int nrhs = nrhs_arr ? max(nrhs_arr[k], 0) : 0;   // (unchecked entries: none for a negative number)
         T *A = dA_array[k];
         T *B = nrhs > 0 ? dB_array[k] : nullptr;
         const int ldb = nrhs > 0 ? lddb_arr[k] : 1;
