@@ -611,15 +611,19 @@ static void launch_panel(int rpt, int m, int n, int j0, int ib, T **dA, int ldda
     else if (rpt == 1)
         MLU_LAUNCH(mlu::KC_PANEL, s, panel_regs_kernel<T, 1, NOPIV><<<nb, PANEL_THREADS, smem, s>>>(
             m, n, j0, ib, dA, ldda, ipiv, info, vs));
-    else if (rpt == 2 && sizeof(T) == 4 && nb > mlu_sm_count())
-        // two CTAs of two rows per thread on an SM (refinement of 512 matrices of order
-        // 512: 516 us of panels, 778 us with one CTA of a row per thread)
-        MLU_LAUNCH(mlu::KC_PANEL, s, panel_regs_kernel<T, 2, NOPIV><<<nb, PANEL_THREADS, smem, s>>>(
-            m, n, j0, ib, dA, ldda, ipiv, info, vs));
-    else if (rpt == 2)
+    else if (rpt == 2) {
+        if constexpr (sizeof(T) == 4) {
+            // two CTAs of two rows per thread on an SM (refinement of 512 matrices of order
+            // 512: 516 us of panels, 778 us with one CTA of a row per thread)
+            if (nb > mlu_sm_count()) {
+                MLU_LAUNCH(mlu::KC_PANEL, s, panel_regs_kernel<T, 2, NOPIV><<<nb, PANEL_THREADS, smem, s>>>(
+                    m, n, j0, ib, dA, ldda, ipiv, info, vs));
+                return;
+            }
+        }
         MLU_LAUNCH(mlu::KC_PANEL, s, panel_regs_kernel<T, 1, NOPIV, 512><<<nb, 512, smem, s>>>(
             m, n, j0, ib, dA, ldda, ipiv, info, vs));
-    else if (rpt == 4)
+    } else if (rpt == 4)
         MLU_LAUNCH(mlu::KC_PANEL, s,
                    panel_regs_kernel<T, (sizeof(T) == 4 ? 2 : 1), NOPIV, 512><<<nb, 512, smem, s>>>(
                        m, n, j0, ib, dA, ldda, ipiv, info, vs));
@@ -676,8 +680,10 @@ magma_int_t blocked_getrf_steps_l(int m, int n, T **dA, int ldda, int **ipiv, in
         mlu_allow_dynamic_smem(panel_regs_kernel<T, 1, false>);
         mlu_allow_dynamic_smem(panel_regs_kernel<T, 1, false, 512>);
         mlu_allow_dynamic_smem(panel_regs_kernel<T, (sizeof(T) == 4 ? 2 : 1), false, 512>);
-        mlu_allow_dynamic_smem(panel_regs_kernel<T, 2, false>);
-        mlu_allow_dynamic_smem(panel_regs_kernel<T, 2, true>);
+        if constexpr (sizeof(T) == 4) {
+            mlu_allow_dynamic_smem(panel_regs_kernel<T, 2, false>);
+            mlu_allow_dynamic_smem(panel_regs_kernel<T, 2, true>);
+        }
         mlu_allow_dynamic_smem(panel_regs_kernel<T, 1, true>);
         mlu_allow_dynamic_smem(panel_regs_kernel<T, 1, true, 512>);
         mlu_allow_dynamic_smem(panel_regs_kernel<T, (sizeof(T) == 4 ? 2 : 1), true, 512>);
