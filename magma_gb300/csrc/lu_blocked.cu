@@ -17,14 +17,14 @@
 //                     band right of the panel): the panel's interchanges, the
 //                     solve L11 U12 = A12 and A22 -= L21 U12 for every row
 //                     tile of the band, U12 kept in shared memory;
-//   right_cols_kernel otherwise, one thread per column right of the panel:
+//   swap_cols_kernel  otherwise, one thread per column right of the panel:
 //     + gemm_kernel   interchanges and U12, then one CTA per 64x64 tile of
 //                     A22 for the update.
 // Every element is updated with one accumulator in increasing k, so the
 // result is bit-identical to the unblocked elimination order.  The
 // interchanges left of each panel are applied after the last step by
 // left_swaps_kernel (one coalesced gather per earlier panel) when the matrix
-// has at most 1024 rows, else by left_tile_kernel in each step.
+// has at most 1024 rows, else by swap_cols_kernel in each step.
 // No workspace and no host synchronisation: every call is stream-ordered and
 // capturable in a CUDA graph.
 #include "common.cuh"
@@ -38,7 +38,6 @@
 namespace mlu {
 
 constexpr int PANEL_THREADS = PANEL_REGS_THREADS;
-constexpr int SWAP_THREADS = 128;
 
 template <typename T, bool NOPIV = false>
 __global__ void __launch_bounds__(PANEL_THREADS)
@@ -98,49 +97,37 @@ __host__ __device__ inline int panel_rows_per_thread(int pm)
     return 0;
 }
 
-// Applies the interchanges of panel [j0, j0+ib) to a SWAP_COLS-column tile left
-// of the panel (matrices too tall for the deferred form, left_swaps_kernel).
-constexpr int SWAP_COLS = 64;
-
-template <typename T>
-__global__ void __launch_bounds__(SWAP_THREADS)
-left_tile_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ipiv_array, StepSizes vs)
-{
-    __shared__ int s_row[2 * PANEL_NB], s_src[2 * PANEL_NB], s_cnt;
-    __shared__ T s_tmp[2 * PANEL_NB * (SWAP_W + 1)];
-    const int mat = blockIdx.y;
-    if (!vs.get(mat, j0, m, n, ldda, ib)) return;
-    const int c0 = blockIdx.x * SWAP_COLS;
-    if (threadIdx.x < 32) build_permutation(ipiv_array[mat], j0, ib, s_row, s_src, &s_cnt);
-    __syncthreads();
-    apply_permutation<T>(dA_array[mat], ldda, c0, min(c0 + SWAP_COLS, j0), s_row, s_src, s_cnt, s_tmp);
-}
-
 // Right of the panel: the interchanges of panel [j0, j0+ib) and U12 = L11^{-1}
 // A12, one thread per column, the column's top block in registers, no barrier
-// after the set-up.  The interchanges as a gather, resolved by each lane running
-// the transpositions backwards: a top row's new content comes from row s_src[k];
-// a row below the top block that an interchange touches ends up holding the
-// original top row s_dsrc[k].  FP64 is bound by the solve's 496 FMAs per column
+// after the set-up.  The blocks from right_blocks on take the columns left of the
+// panel, interchanges only (matrices too tall for the deferred form,
+// left_swaps_kernel), in the same launch, because they wait for nothing that the
+// others do.  The interchanges as a gather, resolved by each lane running the
+// transpositions backwards: a top row's new content comes from row s_src[k]; a row
+// below the top block that an interchange touches ends up holding the original top
+// row s_dsrc[k].  FP64 is bound by the solve's 496 FMAs per column
 // (one FP64 warp instruction per 64 cycles and scheduler), FP32 by the latency of
 // the loads.  n = 512 FP64, 512 matrices: the form with one tile of columns in shared
 // memory (two of four warps solving) took 4260 us per factorisation, this one
 // 3150; n = 1000 FP32, six matrices: 36 us a step, now 12.
-constexpr int RIGHT_COLS = 64;
+constexpr int SWAP_COLS = 64;
 
 template <typename T>
-__global__ void __launch_bounds__(RIGHT_COLS)
-right_cols_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ipiv_array, StepSizes vs, int bj)
+__global__ void __launch_bounds__(SWAP_COLS)
+swap_cols_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ipiv_array, StepSizes vs, int bj,
+                 int right_blocks)
 {
     __shared__ __align__(16) T s_L[PANEL_NB][PANEL_NB];        // [t][i] = L11(i, t)
     __shared__ int s_src[PANEL_NB], s_dst[PANEL_NB], s_dsrc[PANEL_NB];
     const int mat = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
     if (!vs.get(mat, j0, m, n, ldda, ib)) return;
-    n = block_col_end(bj, m, n);                     // right columns end with the block
-    const int c = j0 + ib + blockIdx.x * RIGHT_COLS + tid;
-    if (j0 + ib + (int)blockIdx.x * RIGHT_COLS >= n) return;   // past this matrix's columns
+    const bool left = (int)blockIdx.x >= right_blocks;
+    const int first = left ? ((int)blockIdx.x - right_blocks) * SWAP_COLS : j0 + ib + (int)blockIdx.x * SWAP_COLS;
+    const int c = first + tid;
+    n = left ? j0 : block_col_end(bj, m, n);         // right columns end with the block
+    if (first >= n) return;                          // past this matrix's columns
     T *A = dA_array[mat];
-    for (int e = tid; e < PANEL_NB * PANEL_NB; e += RIGHT_COLS) {
+    for (int e = tid; !left && e < PANEL_NB * PANEL_NB; e += SWAP_COLS) {
         const int i = e % PANEL_NB, t = e / PANEL_NB;
         s_L[t][i] = i < ib && t < ib ? A[j0 + i + (size_t)(j0 + t) * ldda] : T(0);
     }
@@ -179,7 +166,7 @@ right_cols_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int **ip
     // (a panel narrower than 32 has zero coefficients past its width)
 #pragma unroll
     for (int t = 0; t < PANEL_NB; t++) {
-        if (t >= ib) break;
+        if (t >= ib || left) break;
 #pragma unroll
         for (int i = t + 1; i < PANEL_NB; i++) v[i] = Prec<T>::fma_(-s_L[t][i], v[t], v[i]);
     }
@@ -206,8 +193,8 @@ gemm_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int tiles_m, S
 // ---------------------------------------------------------------------------
 // FP32: the step right of the panel in one launch, one CTA per (matrix,
 // BAND_N-column band of columns j0+ib..n).
-//   1. the step's interchanges as a table of touched rows (build_permutation,
-//      warp 0, while the other loads are in flight);
+//   1. the step's interchanges as a table of touched rows (warp 0,
+//      while the other loads are in flight);
 //   2. the band's original top rows (rows j0..j0+ib) and L11 staged in shared
 //      memory, coalesced;
 //   3. the interchanged top rows, i.e. U12 before the solve: a top row's new
@@ -225,9 +212,9 @@ gemm_kernel(int m, int n, int j0, int ib, T **dA_array, int ldda, int tiles_m, S
 //      (always a top row: each interchange k moves row j0+k, which still holds
 //      an original top row, down) takes its value from shared memory, so the
 //      interchanges need no scattered writes.
-// Per element the same operations, in the same order, as right_cols_kernel
+// Per element the same operations, in the same order, as swap_cols_kernel
 // followed by gemm_kernel.  Columns left of the panel are not touched (their
-// interchanges are applied by left_tile_kernel or, after the last step, by
+// interchanges are applied by swap_cols_kernel or, after the last step, by
 // left_swaps_kernel).
 template <typename T>
 __host__ __device__ int blocked_panel_width(int m, int n, int j0);
@@ -659,7 +646,7 @@ static void launch_lu_cta(int m, int n, T **dA, int ldda, int **ipiv, int *info,
 // One step of the blocked factorisation for every matrix: panel at column j0
 // of width ib, interchanges + TRSM, and (when `update`) the trailing update.
 // Right of the panel, band_kernel does all three in one launch (FP32, when the
-// batch gives it at least two CTAs per SM); otherwise right_cols_kernel and
+// batch gives it at least two CTAs per SM); otherwise swap_cols_kernel and
 // gemm_kernel (more, smaller CTAs) do.  `defer_left`: the interchanges left of
 // the panel are left to left_swaps_kernel after the last step.
 // `vsz`: per-matrix sizes of a variable-size batch (m, n = their maxima).
@@ -728,14 +715,11 @@ magma_int_t blocked_getrf_steps_l(int m, int n, T **dA, int ldda, int **ipiv, in
         // one-level n=256 1868 / 1810, n=320 3030 / 3145, n=512 8557 / 9943.
         const bool fused = band_used<T>() && update && bands > 0 && max(m, n) > (bj < 0 ? 288 : 384) &&
                            (long long)bands * nb >= (long long)tune.band_ctas * mlu_sm_count();
-        const int ncl = defer_left ? 0 : (j0 + SWAP_COLS - 1) / SWAP_COLS;
-        const int ncr = fused || rg <= 0 ? 0 : (rg + RIGHT_COLS - 1) / RIGHT_COLS;
-        if (ncl > 0 && ipb != nullptr)
-            MLU_LAUNCH(mlu::KC_SWAP_TRSM, s, left_tile_kernel<T><<<dim3(ncl, nb), SWAP_THREADS, 0, s>>>(
-                m, n, j0, ib, dAb, ldda, ipb, vs));
-        if (ncr > 0)
-            MLU_LAUNCH(mlu::KC_SWAP_TRSM, s, right_cols_kernel<T><<<dim3(ncr, nb), RIGHT_COLS, 0, s>>>(
-                m, n, j0, ib, dAb, ldda, ipb, vs, bj));
+        const int ncl = defer_left || ipb == nullptr ? 0 : (j0 + SWAP_COLS - 1) / SWAP_COLS;
+        const int ncr = fused || rg <= 0 ? 0 : (rg + SWAP_COLS - 1) / SWAP_COLS;
+        if (ncl + ncr > 0)
+            MLU_LAUNCH(mlu::KC_SWAP_TRSM, s, swap_cols_kernel<T><<<dim3(ncl + ncr, nb), SWAP_COLS, 0, s>>>(
+                m, n, j0, ib, dAb, ldda, ipb, vs, bj, ncr));
         if (fused) {
             MLU_LAUNCH(mlu::KC_GEMM, s, band_kernel<<<dim3(bands, nb), BAND_THREADS, band_smem_bytes(), s>>>(
                 m, n, j0, ib, reinterpret_cast<float **>(dAb), ldda, ipb, vs, bj));

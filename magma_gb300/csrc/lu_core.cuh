@@ -17,7 +17,6 @@ namespace mlu {
 
 constexpr int PANEL_NB = 32;          // largest panel width
 constexpr size_t PANEL_SMEM_MAX = 200 * 1024;   // shared memory for one panel
-constexpr int SWAP_W = 32;            // columns per gather/scatter chunk
 constexpr int GEMM_LDU = PANEL_NB + 4; // row stride of the transposed U12 tile in gemm_tile
 
 // Per-matrix sizes for a variable-size batch (device arrays, or all null for a
@@ -337,80 +336,6 @@ __device__ __forceinline__ int panel_factor_regs(int pm, int ib, T *A, int lda, 
 }
 
 // ---------------------------------------------------------------------------
-// Compound permutation of the sequential interchanges k = j0..j0+ib-1 with
-// targets ipiv[k]-1 (1-based ipiv).  Built by warp 0 (threads 0..31 must call
-// it) with ballots over a 64-entry table: s_row[e] is a touched row, s_src[e]
-// the row whose original content ends up there.  The caller synchronises
-// before using the table.
-__device__ __forceinline__ void build_permutation(const int *ipiv, int j0, int ib, int *s_row, int *s_src,
-                                         int *s_cnt)
-{
-    const int lane = threadIdx.x & 31;
-    // all ib targets in one coalesced load, then broadcast by shuffles
-    const int my_target = lane < ib ? ipiv[j0 + lane] - 1 : 0;
-    int cnt = 0;
-    int r0 = -1, r1 = -1, s0 = -1, s1 = -1;   // this lane's entries lane and lane+32
-    for (int k = 0; k < ib; k++) {
-        const int a = j0 + k, b = __shfl_sync(FULL, my_target, k);
-        if (a == b) continue;
-        unsigned fa0 = __ballot_sync(FULL, r0 == a), fa1 = __ballot_sync(FULL, r1 == a);
-        int ia = fa0 ? __ffs(fa0) - 1 : (fa1 ? 32 + __ffs(fa1) - 1 : -1);
-        if (ia < 0) {
-            ia = cnt++;
-            if (lane == (ia & 31)) { if (ia < 32) { r0 = a; s0 = a; } else { r1 = a; s1 = a; } }
-        }
-        unsigned fb0 = __ballot_sync(FULL, r0 == b), fb1 = __ballot_sync(FULL, r1 == b);
-        int ibb = fb0 ? __ffs(fb0) - 1 : (fb1 ? 32 + __ffs(fb1) - 1 : -1);
-        if (ibb < 0) {
-            ibb = cnt++;
-            if (lane == (ibb & 31)) { if (ibb < 32) { r0 = b; s0 = b; } else { r1 = b; s1 = b; } }
-        }
-        const int va = __shfl_sync(FULL, ia < 32 ? s0 : s1, ia & 31);
-        const int vb = __shfl_sync(FULL, ibb < 32 ? s0 : s1, ibb & 31);
-        if (lane == (ia & 31)) { if (ia < 32) s0 = vb; else s1 = vb; }
-        if (lane == (ibb & 31)) { if (ibb < 32) s0 = va; else s1 = va; }
-    }
-    s_row[lane] = r0; s_src[lane] = s0;
-    s_row[lane + 32] = r1; s_src[lane + 32] = s1;
-    if (lane == 0) *s_cnt = cnt;
-}
-
-// Moves the touched rows of columns [c0, c1) of A (ld lda): gather all sources
-// into s_tmp (2*PANEL_NB x (SWAP_W+1)), then scatter, SWAP_W columns at a time.
-// All threads call it; it synchronises internally.
-template <typename T>
-__device__ __forceinline__ void apply_permutation(T *A, int lda, int c0, int c1, const int *s_row, const int *s_src,
-                                  int cnt, T *s_tmp)
-{
-    // rows run fastest across threads, so runs of adjacent rows coalesce;
-    // eight loads per thread in flight before their stores
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    if (cnt == 0) return;
-    for (int cb = c0; cb < c1; cb += SWAP_W) {
-        const int w = min(SWAP_W, c1 - cb);
-        const int total = cnt * w;
-        for (int e0 = tid; e0 < total; e0 += 8 * nthr) {
-            T v[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int e = e0 + u * nthr;
-                if (e < total) v[u] = A[s_src[e % cnt] + (size_t)(cb + e / cnt) * lda];
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int e = e0 + u * nthr;
-                if (e < total) s_tmp[(e % cnt) * (SWAP_W + 1) + e / cnt] = v[u];
-            }
-        }
-        __syncthreads();
-        for (int e = tid; e < cnt * w; e += nthr) {
-            const int pr = e % cnt, c = e / cnt;
-            A[s_row[pr] + (size_t)(cb + c) * lda] = s_tmp[pr * (SWAP_W + 1) + c];
-        }
-        __syncthreads();
-    }
-}
-
 // One BM x BN tile of A22 -= L21 * U12 with rows from r0 and columns from c0
 // (rows >= m or columns >= n skipped).  L21 columns j0..j0+ib, U12 rows
 // j0..j0+ib.  sL, sU: PANEL_NB x BM and BN x GEMM_LDU T.  Called by exactly
