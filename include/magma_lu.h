@@ -773,16 +773,21 @@ magma_int_t magma_svbatched_tuning_set(const magma_int_t *nb, const magma_int_t 
  * (control/get_batched_crossover.cpp:300-342, 918-928;
  * control/get_batched_gemm_decision.cpp:233-253).  One table per precision,
  * six size bins of max(m, n): <= 64, 128, 256, 512, 1024, larger.  Entries:
- *   two_level[b]  FP32: 1 = 128-column blocks with one rank-128 update right of
- *                 each, 0 = a rank-32 update after every 32-column panel;
+ *   two_level[b]  FP32: 1 permits 128-column blocks with one rank-128 update right
+ *                 of each, which run for n > 176 when the batch gives every SM one
+ *                 of those updates; 0 = a rank-32 update after every 32-column
+ *                 panel, always;
  *   band_ctas[b]  FP32: the fused band kernel when a step gives at least this
- *                 many CTAs per SM (1, 2 or 4);
- *   tile64[b]     FP64: 1 = 64 x 64 update tiles, 0 = 32 x 32.
+ *                 many CTAs per SM (1, 2 or 4) and max(m, n) is above 288 (above
+ *                 384 with two levels);
+ *   tile64[b]     FP64: 1 = 64 x 64 update tiles, 0 = 32 x 32, where several CTAs
+ *                 update one matrix (small matrices are factored by one CTA each).
  * Every setting gives bit-identical results; only the time changes.
  *
  * magma_?getrf_batched_autotune: times the candidates of every bin up to max_n
  * on `batch` trial matrices on `queue`'s device (allocates them, synchronises)
- * and installs the fastest.  Must not run beside other calls of this library.
+ * and installs the fastest.  Settings that launch the same kernels for a bin's
+ * trial are one candidate, and a bin with one candidate keeps its entry.  Must not run beside other calls of this library.
  * Errors: -1 max_n < 0, -2 batch < 1, -3 no queue, MAGMA_ERR_DEVICE_ALLOC.
  * magma_?getrf_batched_tuning_get / _set: read or replace the table (six
  * entries per array); _set returns -1 / -2 / -3 for a bad entry.

@@ -33,6 +33,7 @@
 #include "solve_core.cuh"
 #include "lu_cta.cuh"
 
+#include <string>
 #include <type_traits>
 
 namespace mlu {
@@ -643,6 +644,22 @@ static void launch_lu_cta(int m, int n, T **dA, int ldda, int **ipiv, int *info,
     MLU_LAUNCH(mlu::KC_PANEL, s, lu_cta_kernel<T, NT><<<batch, NT, cta_lu_smem<T>(m, n, min(m, CTA_NB)), s>>>(m, n, dA, ldda, ipiv, info));
 }
 
+// Whether the fused band kernel takes the update of a step with rg columns right of the
+// panel.  It pays for its set-up (five barriers, two CTAs per SM) on long columns only:
+// batch 1000, getrf us with it / with the separate kernels,
+// two-level n=200 1204 / 1065, n=320 2708 / 2647, n=512 6274 / 6303;
+// one-level n=256 1868 / 1810, n=320 3030 / 3145, n=512 8557 / 9943.
+template <typename T>
+static bool step_fused(int m, int n, int rg, int bj, int nb, int band_ctas)
+{
+    const int bands = rg > 0 ? (rg + BAND_N - 1) / BAND_N : 0;
+    return band_used<T>() && bands > 0 && max(m, n) > (bj < 0 ? 288 : 384) &&
+           (long long)bands * nb >= (long long)band_ctas * mlu_sm_count();
+}
+
+// Whether the update of an rm x rn trailing block runs on 64 x 64 tiles.
+static bool step_tile64(bool tile64, int rm, int rn) { return tile64 && rm > 32 && rn > 32; }
+
 // One step of the blocked factorisation for every matrix: panel at column j0
 // of width ib, interchanges + TRSM, and (when `update`) the trailing update.
 // Right of the panel, band_kernel does all three in one launch (FP32, when the
@@ -709,12 +726,7 @@ magma_int_t blocked_getrf_steps_l(int m, int n, T **dA, int ldda, int **ipiv, in
         // whose last panel is narrower than ib has up to ib - 1 more of them
         const int rg = vs.m_arr ? block_col_end(bj, m, n) - j0 - 1 : rn;
         const int bands = rg > 0 ? (rg + BAND_N - 1) / BAND_N : 0;
-        // The fused band kernel pays for its set-up (five barriers, two CTAs per SM) on
-        // long columns only: batch 1000, getrf us with it / with the separate kernels,
-        // two-level n=200 1204 / 1065, n=320 2708 / 2647, n=512 6274 / 6303;
-        // one-level n=256 1868 / 1810, n=320 3030 / 3145, n=512 8557 / 9943.
-        const bool fused = band_used<T>() && update && bands > 0 && max(m, n) > (bj < 0 ? 288 : 384) &&
-                           (long long)bands * nb >= (long long)tune.band_ctas * mlu_sm_count();
+        const bool fused = update && step_fused<T>(m, n, rg, bj, nb, tune.band_ctas);
         const int ncl = defer_left || ipb == nullptr ? 0 : (j0 + SWAP_COLS - 1) / SWAP_COLS;
         const int ncr = fused || rg <= 0 ? 0 : (rg + SWAP_COLS - 1) / SWAP_COLS;
         if (ncl + ncr > 0)
@@ -724,7 +736,7 @@ magma_int_t blocked_getrf_steps_l(int m, int n, T **dA, int ldda, int **ipiv, in
             MLU_LAUNCH(mlu::KC_GEMM, s, band_kernel<<<dim3(bands, nb), BAND_THREADS, band_smem_bytes(), s>>>(
                 m, n, j0, ib, reinterpret_cast<float **>(dAb), ldda, ipb, vs, bj));
         } else if (update && rm > 0 && rn > 0) {
-            if (!tune.tile64 || rm <= 32 || rn <= 32) {
+            if (!step_tile64(tune.tile64, rm, rn)) {
                 // a thin trailing block: 32 x 32 tiles, so that no FMA of a
                 // 64 x 64 tile runs on padding (each costs full FP64 issue slots)
                 const int tiles_m = (rm + 31) / 32, tiles_n = (rn + 31) / 32;
@@ -804,9 +816,14 @@ static bool outer_blocked(int m, int n)
 // and when enough columns lie right of the first block (b=1000: n=144 732 / 572,
 // n=200 1065 / 1153).
 template <typename T>
+static bool outer_worthwhile(int m, int n, int batch)
+{
+    return outer_blocked_shape<T>(m, n) && n > 176 && (long long)batch * mlu_ceildiv(n - OUTER_NB, OUTER_NB) >= mlu_sm_count();
+}
+template <typename T>
 static bool outer_blocked(int m, int n, int batch)
 {
-    return outer_blocked<T>(m, n) && n > 176 && (long long)batch * mlu_ceildiv(n - OUTER_NB, OUTER_NB) >= mlu_sm_count();
+    return outer_worthwhile<T>(m, n, batch) && outer_blocked<T>(m, n);
 }
 
 // Steps of the two-level blocked factorisation: per 128-column block, its
@@ -876,6 +893,26 @@ static bool one_cta_per_matrix(int n, int batch)
     return n <= 112 || (n <= CTA_MAX_N && 4LL * batch >= 3LL * mlu_sm_count());
 }
 
+// The kernels that a factorisation of `batch` matrices of order n launches under the
+// tuning entries c, one letter per step: entries with the same form are the same code.
+template <typename T>
+std::string fixed_form(int n, int batch, const FixedChoice &c)
+{
+    if (one_cta_per_matrix<T>(n, batch)) return "c";
+    const bool two = c.two_level && outer_worthwhile<T>(n, n, batch);
+    const int nb = min(batch, (int)MLU_MAX_GRID_Y);
+    std::string f = two ? "2" : "1";
+    for (int j0 = 0; j0 < n;) {
+        const int ib = blocked_panel_width<T>(n, n, j0), bj = two ? j0 / OUTER_NB * OUTER_NB : -1;
+        const int rm = n - j0 - ib, rn = block_col_end(bj, n, n) - j0 - ib;
+        f += rn <= 0 ? '-' : step_fused<T>(n, n, rn, bj, nb, c.band_ctas) ? 'b' : step_tile64(c.tile64, rm, rn) ? 'L' : 's';
+        j0 += ib;
+    }
+    return f;
+}
+template std::string fixed_form<double>(int, int, const FixedChoice &);
+template std::string fixed_form<float>(int, int, const FixedChoice &);
+
 template <typename T>
 magma_int_t blocked_getrf(int m, int n, T **dA, int ldda, int **ipiv, int *info, int batch,
                           magma_queue_t q)
@@ -921,7 +958,6 @@ magma_int_t blocked_getrf_two_level(int m, int n, float **dA, int ldda, int **ip
                                       outer, ctx);
 }
 bool two_level_applies(int m, int n) { return outer_blocked<float>(m, n); }
-bool two_level_possible(int m, int n) { return outer_blocked_shape<float>(m, n); }
 
 template int blocked_panel_width<float>(int, int, int);
 template magma_int_t blocked_getrf_steps<float>(int, int, float **, int, int **, int *, int,

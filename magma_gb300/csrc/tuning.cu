@@ -7,12 +7,15 @@
 // the choices that matter on GB300 are a table per precision and size bin of
 // max(m, n) (<= 64, 128, 256, 512, 1024, larger):
 //   two_level   FP32: 128-column blocks with one rank-128 update right of each
-//               (lu_outer.cu), or a rank-32 update after every panel;
+//               (lu_outer.cu) where the order and the batch are worth it
+//               (outer_worthwhile in lu_blocked.cu), or a rank-32 update after
+//               every panel always;
 //   band_ctas   FP32: the fused band kernel when the step gives at least this
-//               many CTAs per SM (1, 2 or 4), else separate interchange and
-//               update kernels;
+//               many CTAs per SM (1, 2 or 4) and the columns are long enough
+//               (step_fused), else separate interchange and update kernels;
 //   tile64      FP64: 64 x 64 update tiles (32 x 32 for thin trailing blocks),
-//               or 32 x 32 always.
+//               or 32 x 32 always, in the step kernels (not where one CTA takes
+//               a whole matrix, one_cta_per_matrix).
 // Every choice performs the same operations on every element in the same
 // order, so tuning never changes a result.  magma_?getrf_batched_autotune times
 // the candidates on the device and installs the fastest;
@@ -29,6 +32,7 @@
 #include <stdlib.h>
 #include <string.h>
 #include <string>
+#include <vector>
 
 extern "C" magma_int_t magma_dvbatched_tuning_get(magma_int_t *nb, magma_int_t *tile);
 extern "C" magma_int_t magma_svbatched_tuning_get(magma_int_t *nb, magma_int_t *tile);
@@ -109,12 +113,35 @@ __global__ void tune_arrays_kernel(int k, int n, T *A, int *P, T **dA, int **dP)
 template <typename T>
 magma_int_t blocked_getrf(int m, int n, T **dA, int ldda, int **ipiv, int *info, int batch,
                           magma_queue_t q);
-bool two_level_possible(int m, int n);
+template <typename T> std::string fixed_form(int n, int batch, const FixedChoice &c);
 
-// Times every candidate of every bin up to max_n on `batch` trial matrices of
+// The settings of bin b that launch different kernels for `batch` matrices of order n
+// (fixed_form), the installed one first; among settings that launch the same the one
+// that keeps more of the installed entries.
+template <typename T>
+static std::vector<FixedChoice> fixed_candidates(const FixedTune &t, int b, int n, int batch)
+{
+    std::vector<FixedChoice> out;
+    std::vector<std::string> forms;
+    const bool fp64 = sizeof(T) == 8;
+    const int bcs[4] = {t.band_ctas[b], 1, 2, 4};
+    for (int i = 0; i < (fp64 ? 1 : 2); i++)
+        for (int bc : bcs)
+            for (int k = 0; k < (fp64 ? 2 : 1); k++) {
+                const FixedChoice c = {(t.two_level[b] != 0) != (i != 0), fp64 ? (int)t.band_ctas[b] : bc, (t.tile64[b] != 0) != (k != 0)};
+                const std::string f = fixed_form<T>(n, batch, c);
+                if (std::find(forms.begin(), forms.end(), f) != forms.end()) continue;
+                forms.push_back(f);
+                out.push_back(c);
+            }
+    return out;
+}
+
+// Times the candidates of every bin up to max_n on `batch` trial matrices of
 // three quarters of the bin's largest order (max_n itself for the last bin);
-// installs the fastest per bin.  Other calls must not run meanwhile: the trials
-// run through the shared table.
+// installs the fastest per bin.  A bin whose settings all launch the same kernels for
+// that order and batch keeps its entry, untimed: it may matter for another batch.
+// Other calls must not run meanwhile: the trials run through the shared table.
 template <typename T>
 static magma_int_t fixed_autotune(int max_n, int batch, magma_queue_t q)
 {
@@ -137,6 +164,8 @@ static magma_int_t fixed_autotune(int max_n, int batch, magma_queue_t q)
         // at most ~1 GB of trial matrices
         const int k = (int)std::max<size_t>(
             1, std::min<size_t>((size_t)batch, ((size_t)1 << 30) / ((size_t)n * n * sizeof(T))));
+        const std::vector<FixedChoice> cand = fixed_candidates<T>(t, b, n, k);
+        if (cand.size() < 2) continue;
         T *A = nullptr, **dA = nullptr;
         int *P = nullptr, **dP = nullptr, *info = nullptr;
         if (device_malloc((void **)&A, (size_t)k * n * n * sizeof(T)) != cudaSuccess ||
@@ -149,22 +178,13 @@ static magma_int_t fixed_autotune(int max_n, int batch, magma_queue_t q)
         }
         if (rc == MAGMA_SUCCESS) {
             MLU_LAUNCH(mlu::KC_OTHER, s, tune_arrays_kernel<T><<<(k + 255) / 256, 256, 0, s>>>(k, n, A, P, dA, dP));
-            // candidates: (two_level, band_ctas, tile64)
-            int cand[12][3], nc = 0;
-            if (fp64) {
-                for (int t64 = 0; t64 < 2; t64++) { cand[nc][0] = 1; cand[nc][1] = 2; cand[nc][2] = t64; nc++; }
-            } else {
-                const int tl_max = two_level_possible(n, n) ? 1 : 0;
-                for (int tl = 0; tl <= tl_max; tl++)
-                    for (int bc : {1, 2, 4}) { cand[nc][0] = tl; cand[nc][1] = bc; cand[nc][2] = 1; nc++; }
-            }
             float best = -1.f;
-            int bi = 0;
-            for (int c = 0; c < nc && rc == MAGMA_SUCCESS; c++) {
+            size_t bi = 0;
+            for (size_t c = 0; c < cand.size() && rc == MAGMA_SUCCESS; c++) {
                 FixedTune trial = t;
-                trial.two_level[b] = (unsigned char)cand[c][0];
-                trial.band_ctas[b] = (unsigned char)cand[c][1];
-                trial.tile64[b] = (unsigned char)cand[c][2];
+                trial.two_level[b] = cand[c].two_level;
+                trial.band_ctas[b] = (unsigned char)cand[c].band_ctas;
+                trial.tile64[b] = cand[c].tile64;
                 fixed_put(fp64, trial);
                 float tmin = -1.f;
                 for (int rep = 0; rep < 2 && rc == MAGMA_SUCCESS; rep++) {
@@ -187,9 +207,9 @@ static magma_int_t fixed_autotune(int max_n, int batch, magma_queue_t q)
                     bi = c;
                 }
             }
-            t.two_level[b] = (unsigned char)cand[bi][0];
-            t.band_ctas[b] = (unsigned char)cand[bi][1];
-            t.tile64[b] = (unsigned char)cand[bi][2];
+            t.two_level[b] = cand[bi].two_level;
+            t.band_ctas[b] = (unsigned char)cand[bi].band_ctas;
+            t.tile64[b] = cand[bi].tile64;
         }
         cudaFree(A); cudaFree(P); cudaFree(dA); cudaFree(dP); cudaFree(info);
     }
