@@ -739,20 +739,22 @@ magma_int_t magma_sposv_batched(magma_uplo_t uplo, magma_int_t n, magma_int_t nr
  * (control/get_batched_crossover.cpp:300-342, 918-928).
  *
  * The persistent kernel of magma_?getrf_vbatched / magma_?gesv_vbatched picks,
- * per matrix, a panel width (nb: 8, 16 or 32) and a trailing-update tile
- * (tile: 0 = 64x64, 1 = 32x64, 2 = 32x32) from a table indexed by the size bin
- * of max(m, n): <= 16, 32, 64, 128, 256, 512, 1024, larger (8 entries).  No
- * choice changes a result bit: every element receives the same updates in the
+ * per matrix, a panel width (nb: 8, 16 or 32; 32 runs as 16) and the elements
+ * each thread updates (tile: 0 or 1 = 4x4, 2 = 2x2) from a table indexed by the
+ * size bin of max(m, n): <= 16, 32, 64, 128, 256, 512, 1024, larger (8 entries).
+ * No choice changes a result bit: every element receives the same updates in the
  * same order.
  *
  * Batches whose largest matrix exceeds 256 do not use the table: they run the
  * per-step kernels of the fixed-size path with per-matrix sizes (several CTAs
  * per matrix and step).
  *
- * magma_?getrf_vbatched_autotune: times every (nb in {16, 32}) x (tile)
- * candidate on `queue`'s device for each bin up to max_n (bins above 256 are
- * not timed), installs the fastest in the table of that precision and returns
- * the table in nb[8], tile[8] (either may be NULL).  Allocates its trial
+ * magma_?getrf_vbatched_autotune: times the four choices that run different
+ * code (panels of 8 or 16 columns, 4x4 or 2x2 elements) on `queue`'s device for
+ * each bin up to max_n (bins above 256 are not timed), installs the fastest in
+ * the table of that precision -- an installed entry that runs the same code as
+ * the fastest stays as it is -- and returns the table in nb[8], tile[8] (either
+ * may be NULL).  Allocates its trial
  * batches and synchronises the queue.  max_n = 0 only returns the table.
  * Errors: -1 max_n < 0, -4 no queue, MAGMA_ERR_DEVICE_ALLOC.
  *

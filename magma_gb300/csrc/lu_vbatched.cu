@@ -208,7 +208,7 @@ magma_int_t vb_getrs_run(bool trans, const int *n, const int *nrhs, int max_n, i
                          magma_queue_t q);
 
 // Tuning tables in use (one per precision), set by magma_?vbatched_tuning_set
-// or the autotuner.  Defaults: the autotuner's choices on GB300.
+// or the autotuner.  Defaults: panels of 16 columns (32 runs as 16), 4 x 4 elements.
 static std::mutex g_tune_mu;
 static VbTune g_tune[2] = {
     {{32, 32, 32, 32, 32, 32, 32, 32}, {0, 0, 0, 0, 0, 0, 0, 0}},   // double
@@ -532,7 +532,6 @@ __global__ void vb_trial_arrays_kernel(int k, int n, T *A, int *P, T **dA, int *
     dld[i] = n;
 }
 
-static const int VB_TUNE_NB[] = {16, 32};
 constexpr int VB_TUNE_MAX_N = VB_PERSISTENT_MAX;   // larger bins do not use the table
 
 template <typename T>
@@ -581,8 +580,13 @@ static magma_int_t vb_autotune(int max_n, magma_queue_t q, VbTune *out)
                 k, n, A, P, dA, dP, dn, dld));
             float best = -1.f;
             int best_nb = t.nb[b], best_tile = t.tile[b];
-            for (int nbw : VB_TUNE_NB) {
-                for (int tile = 0; tile < VB_TILE_COUNT && rc == MAGMA_SUCCESS; tile++) {
+            // the settings that run different code: a panel width of 8 or 16, 4 x 4 or 2 x 2
+            // elements per thread; of equal ones the installed entry
+            const int nbs[2] = {best_nb, min(best_nb, CTA_NB) == 8 ? CTA_NB : 8};
+            const int tiles[2] = {best_tile, best_tile == VB_TILE_32x32 ? (int)VB_TILE_64x64 : (int)VB_TILE_32x32};
+            for (int nbw : nbs) {
+                for (int tile : tiles) {
+                    if (rc != MAGMA_SUCCESS) break;
                     VbTune trial = t;
                     trial.nb[b] = (unsigned char)nbw;
                     trial.tile[b] = (unsigned char)tile;
