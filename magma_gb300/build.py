@@ -77,9 +77,9 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> Path:
 def build_bounds_check(force: bool = False) -> Path:
     """The bounds-check build (-DMLU_BOUNDS_CHECK): the same sources with every
     instrumented global access checked against its operand's logical extent, the
-    first violation recorded in a device word (mlu_bounds_check_read).  Separate
-    objects and library (libmagma_lu_bc.so); relocatable device code, so that
-    every translation unit records into the one word.  Its function-local statics (the
+    first violation recorded on the device (mlu_bounds_check_read).  Separate
+    objects and library (libmagma_lu_bc.so), compiled with the normal library's flags
+    otherwise.  Its function-local statics (the
     per-device caches of kernel attributes) are ordinary weak symbols bound inside the
     library (-fno-gnu-unique, -Bsymbolic): as GNU-unique symbols the dynamic linker would
     merge them with the normal library's in a process that loads both, and one library's
@@ -87,11 +87,11 @@ def build_bounds_check(force: bool = False) -> Path:
     if not force and LIB_BC.exists() and all(p.stat().st_mtime <= LIB_BC.stat().st_mtime for p in _deps()):
         return LIB_BC
     BUILD_BC.mkdir(exist_ok=True)
-    extra = ["-rdc=true", "-DMLU_BOUNDS_CHECK", "-Xcompiler", "-fno-gnu-unique"]
+    extra = ["-DMLU_BOUNDS_CHECK", "-Xcompiler", "-fno-gnu-unique"]
     srcs = sources()
     with cf.ThreadPoolExecutor(max_workers=min(len(srcs), os.cpu_count() or 4)) as ex:
         objs = list(ex.map(lambda s: _compile(s, extra, BUILD_BC), srcs))
-    _link(objs, LIB_BC, ["-rdc=true", "-Xlinker", "-Bsymbolic"])
+    _link(objs, LIB_BC, ["-Xlinker", "-Bsymbolic"])
     return LIB_BC
 
 

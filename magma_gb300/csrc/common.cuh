@@ -156,8 +156,31 @@ __device__ __forceinline__ T shfl(T v, int src) { return __shfl_sync(FULL, v, sr
 // the logical m x n operand; otherwise it records the first violation (site,
 // r, c) in a device word, counts it, and is false, so that the caller skips the
 // access.  In the normal build it is the constant true and costs nothing.
+// Every translation unit has a record of its own (bc_record), which its object registers
+// with the reader (runtime.cu): so the build needs no relocatable device code and its
+// kernels are compiled as the normal library's are, but for the checks.
 #ifdef MLU_BOUNDS_CHECK
-__device__ void bc_fail(int site, long long r, long long c);
+struct BcRecord {
+    unsigned long long first, count;   // site << 48 | row << 24 | column of the first violation; violations
+};
+static __device__ BcRecord g_bc_record;
+static __device__ __noinline__ void bc_fail(int site, long long r, long long c)
+{
+    const unsigned long long rec = ((unsigned long long)(site & 0xffff) << 48) |
+                                   (((unsigned long long)r & 0xffffffull) << 24) |
+                                   ((unsigned long long)c & 0xffffffull);
+    atomicCAS(&g_bc_record.first, 0ull, rec);
+    atomicAdd(&g_bc_record.count, 1ull);
+}
+void bc_register(cudaError_t (*address)(void **));
+namespace {
+struct BcRegister {
+    BcRegister()
+    {
+        bc_register([](void **p) { return cudaGetSymbolAddress(p, g_bc_record); });
+    }
+} bc_register_this_unit;
+}  // namespace
 #define MLU_BC2(r, c, m, n, site)                                                         \
     (((unsigned long long)(long long)(r) < (unsigned long long)(long long)(m) &&         \
       (unsigned long long)(long long)(c) < (unsigned long long)(long long)(n))            \

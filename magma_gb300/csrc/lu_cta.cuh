@@ -114,15 +114,13 @@ __device__ __forceinline__ void cta_step(T (&a)[CTA_NB], T l, const T *rest, Cta
 // `i` (a permutation of the thread index by whole warps) per thread.  On return
 // sP[j * ldp + i] and Ap hold it in pivoted order, s.ipiv / slot / dst are set
 // (visible to all threads) and the return value is the 1-based column of the
-// first zero pivot, or 0, in every thread with a row.  top: room for the panel's U rows
-// (volatile: without it the bounds-check build, which is relocatable code, came out of
-// the compiler with one column of the first update taken from another).
+// first zero pivot, or 0, in every thread with a row.  top: room for the panel's U rows.
 //
 // A row's remaining columns sit in its thread's registers with the current one
 // first, so that the column loop stays a loop.  A column that is done leaves for
 // sP, in physical row order until the end.
 template <typename T, int NCH>
-__device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, int ldp, volatile T *top, CtaPanel<T, NCH> &s, int i)
+__device__ __forceinline__ int cta_panel(int pm, int ib, T *Ap, int lda, T *sP, int ldp, T *top, CtaPanel<T, NCH> &s, int i)
 {
     const int lane = i & 31, chunk = i >> 5;
     const int nch = (pm + 31) >> 5;                      // 32-row blocks
@@ -262,7 +260,7 @@ __device__ __forceinline__ void cta_column(T *col, int pm, int ib, const T *sP, 
     for (int q = 0; q < CTA_NB; q++)
         if (FULL || q < ib) {
             col[q] = v[q];
-            if (SOLVE) sU[q * ldu] = v[q];
+            if (SOLVE && MLU_BC2(q, 0, CTA_NB, ldu, 708)) sU[q * ldu] = v[q];
         }
 }
 
@@ -280,7 +278,10 @@ __device__ __forceinline__ void cta_update(T *A22, int lda, int rm, int rn, int 
 #pragma unroll
         for (int b = 0; b < M; b++)
 #pragma unroll
-            for (int a = 0; a < M; a++) acc[b][a] = (r + a < rm && c + b < rn) ? p[a + (size_t)b * lda] : T(0);
+            for (int a = 0; a < M; a++)
+                acc[b][a] = (r + a < rm && c + b < rn && MLU_BC2(r + a, c + b, rm, rn, 705)) ? p[a + (size_t)b * lda] : T(0);
+        // (a block reads L21 and U12 up to its fourth row and column)
+        if (!MLU_BC2(r + M - 1, c + M - 1, ldp - ib, ldu, 706)) continue;
         for (int k0 = 0; k0 < ib; k0 += 8) {
 #pragma unroll 2
             for (int k = 0; k < 8; k++) {
@@ -297,7 +298,7 @@ __device__ __forceinline__ void cta_update(T *A22, int lda, int rm, int rn, int 
         for (int b = 0; b < M; b++)
 #pragma unroll
             for (int a = 0; a < M; a++)
-                if (r + a < rm && c + b < rn) p[a + (size_t)b * lda] = acc[b][a];
+                if (r + a < rm && c + b < rn && MLU_BC2(r + a, c + b, rm, rn, 707)) p[a + (size_t)b * lda] = acc[b][a];
     }
 }
 

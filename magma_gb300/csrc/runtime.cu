@@ -10,6 +10,7 @@
 #include "trace.cuh"
 #include <atomic>
 #include <stdlib.h>
+#include <vector>
 
 namespace {
 std::atomic<int> g_fail_allocs{0};   // allocations still to fail (fault injection for tests)
@@ -215,34 +216,29 @@ extern "C" magma_int_t magma_lu_set_pointers(void **output_arrays, magma_int_t a
 }
 
 #ifdef MLU_BOUNDS_CHECK
-// The bounds-check build's record: the first violation (site << 48 | row << 24
-// | column, each clipped to 24 bits) and the number of violations.
 namespace mlu {
-__device__ unsigned long long g_bc_first;
-__device__ unsigned long long g_bc_count;
-__device__ void bc_fail(int site, long long r, long long c)
+using BcAddress = cudaError_t (*)(void **);
+static std::vector<BcAddress> &bc_records()
 {
-    const unsigned long long rec = ((unsigned long long)(site & 0xffff) << 48) |
-                                   (((unsigned long long)r & 0xffffffull) << 24) |
-                                   ((unsigned long long)c & 0xffffffull);
-    atomicCAS(&g_bc_first, 0ull, rec);
-    atomicAdd(&g_bc_count, 1ull);
+    static std::vector<BcAddress> v;             // (filled by static constructors, in any order)
+    return v;
 }
+void bc_register(BcAddress address) { bc_records().push_back(address); }
 }  // namespace mlu
 
-// Reads the record (first violation, count) and, with reset != 0, clears it.
-// Exported by the bounds-check build only.
+// Reads the records of all translation units (a first violation of one of them, the
+// number in all) and, with reset != 0, clears them.  Exported by the bounds-check build only.
 extern "C" int mlu_bounds_check_read(unsigned long long *first, unsigned long long *count, int reset)
 {
     if (cudaDeviceSynchronize() != cudaSuccess) return -1;
-    if (cudaMemcpyFromSymbol(first, mlu::g_bc_first, sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMemcpyFromSymbol(count, mlu::g_bc_count, sizeof(unsigned long long)) != cudaSuccess)
-        return -1;
-    if (reset) {
-        const unsigned long long z = 0;
-        if (cudaMemcpyToSymbol(mlu::g_bc_first, &z, sizeof z) != cudaSuccess ||
-            cudaMemcpyToSymbol(mlu::g_bc_count, &z, sizeof z) != cudaSuccess)
-            return -1;
+    *first = *count = 0;
+    for (mlu::BcAddress address : mlu::bc_records()) {
+        void *p = nullptr;
+        mlu::BcRecord r;
+        if (address(&p) != cudaSuccess || cudaMemcpy(&r, p, sizeof r, cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
+        if (*count == 0) *first = r.first;
+        *count += r.count;
+        if (reset && cudaMemset(p, 0, sizeof r) != cudaSuccess) return -1;
     }
     return 0;
 }

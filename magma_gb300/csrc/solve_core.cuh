@@ -60,13 +60,13 @@ template <> struct Diag<float> {
 // Block [t0, t0 + tb) of the factor by cp.async, all threads.  Rows and columns
 // past tb are set to zero.
 template <typename T, bool CT>
-__device__ __forceinline__ void stage_diag(const T *A, int lda, int t0, int tb, Diag<T> &D)
+__device__ __forceinline__ void stage_diag(int n, const T *A, int lda, int t0, int tb, Diag<T> &D)
 {
     constexpr int LD = Diag<T>::LD;
     for (int e = threadIdx.x; e < 32 * 32; e += blockDim.x) {
         const int r = e & 31, c = e >> 5;
         T *dst = D.d + (sizeof(T) == 4 && !CT ? c * LD + r : r * LD + c);
-        const bool in = r < tb && c < tb;
+        const bool in = r < tb && c < tb && MLU_BC2(t0 + r, t0 + c, n, n, 801);
         cp_async_elem<sizeof(T)>(dst, in ? A + t0 + r + (size_t)(t0 + c) * lda : A, in);
     }
     cp_async_commit();
@@ -76,8 +76,9 @@ __device__ __forceinline__ void stage_diag(const T *A, int lda, int t0, int tb, 
 // block, of which tb exist: c(i, t) = A(i, t), or A(t, i) with CT.  Columns past
 // tb read as zero.  `vec`: 16-byte loads along t are aligned (CT).
 template <typename T, bool CT, int LW>
-__device__ __forceinline__ void load_coefs(T (&l)[LW], const T *A, int lda, int i, int t0, int tb, bool vec)
+__device__ __forceinline__ void load_coefs(T (&l)[LW], int n, const T *A, int lda, int i, int t0, int tb, bool vec)
 {
+    if (tb > 0 && (!MLU_BC2(i, t0, n, n, 802) || !MLU_BC2(i, t0 + min(tb, LW) - 1, n, n, 803))) tb = 0;
     const T *p = CT ? A + (size_t)i * lda + t0 : A + i + (size_t)t0 * lda;
     const size_t step = CT ? 1 : lda;
     if (tb < LW) {
@@ -335,7 +336,7 @@ __device__ __forceinline__ void tri_sweep(int n, const T *A, int lda, T *sB, int
     constexpr int H0 = ASC ? 0 : 32 - LW;            // the half (or all) of a block's columns used first
     {
         const int t0 = ASC ? 0 : 32 * (nb - 1);
-        stage_diag<T, CT>(A, lda, t0, min(32, n - t0), D);
+        stage_diag<T, CT>(n, A, lda, t0, min(32, n - t0), D);
     }
     for (int s = 0; s < nb; s++) {
         const int t0 = 32 * (ASC ? s : nb - 1 - s), tb = min(32, n - t0);
@@ -348,7 +349,7 @@ __device__ __forceinline__ void tri_sweep(int n, const T *A, int lda, T *sB, int
         // the first task's coefficients are in flight during D: in the warps that do
         // not take part in it and, where there are registers for it (FP64), in all
         const bool early = (sizeof(T) == 8 && LW == 32) || (sizeof(T) == 4 && warp > 0);
-        if (early && w0 < ntask) load_coefs<T, CT, LW>(l, A, lda, min(i, rend - 1), t0 + H0, tb - H0, vec);
+        if (early && w0 < ntask) load_coefs<T, CT, LW>(l, n, A, lda, min(i, rend - 1), t0 + H0, tb - H0, vec);
         cp_async_wait<0>();
         __syncthreads();                          // the diagonal block, and the previous update
         T *x = sB + t0;
@@ -366,11 +367,11 @@ __device__ __forceinline__ void tri_sweep(int n, const T *A, int lda, T *sB, int
         } else if (warp == 0) {
             diag_cols<ASC, UNIT>(D, x, ldx, nr, tb);
         }
-        if (!early && w0 < ntask) load_coefs<T, CT, LW>(l, A, lda, min(i, rend - 1), t0 + H0, tb - H0, vec);
+        if (!early && w0 < ntask) load_coefs<T, CT, LW>(l, n, A, lda, min(i, rend - 1), t0 + H0, tb - H0, vec);
         __syncthreads();
         if (s + 1 < nb) {
             const int u0 = 32 * (ASC ? s + 1 : nb - 2 - s);
-            stage_diag<T, CT>(A, lda, u0, min(32, n - u0), D);
+            stage_diag<T, CT>(n, A, lda, u0, min(32, n - u0), D);
         }
         for (int task = w0; task < ntask;) {
             const int c0 = ng == 1 ? 0 : (task % ng) * CG;
@@ -382,7 +383,7 @@ __device__ __forceinline__ void tri_sweep(int n, const T *A, int lda, T *sB, int
 #pragma unroll
             for (int h = 0; h < 32 / LW; h++) {
                 const int o = ASC ? h * LW : 32 - LW - h * LW;
-                if (h > 0) load_coefs<T, CT, LW>(l, A, lda, min(i, rend - 1), t0 + o, tb - o, vec);
+                if (h > 0) load_coefs<T, CT, LW>(l, n, A, lda, min(i, rend - 1), t0 + o, tb - o, vec);
                 if (CG > 1 && sizeof(T) == 8 && c0 + 1 >= nr) {
                     T one[1] = {acc[0]};           // a last odd column alone
                     update_row<T, 1, ASC, LW>(one, l, xs + o, ldx, tb - o);
@@ -394,12 +395,12 @@ __device__ __forceinline__ void tri_sweep(int n, const T *A, int lda, T *sB, int
             if (i < rend) {
 #pragma unroll
                 for (int q = 0; q < CG; q++)
-                    if (c0 + q < nr) xr[(size_t)q * ldx] = acc[q];
+                    if (c0 + q < nr && MLU_BC2(i, c0 + q, n, nr, 807)) xr[(size_t)q * ldx] = acc[q];
             }
             task += nw;
             if (task < ntask) {
                 i = rbase + 32 * (ng == 1 ? task : task / ng) + lane;
-                load_coefs<T, CT, LW>(l, A, lda, min(i, rend - 1), t0 + H0, tb - H0, vec);
+                load_coefs<T, CT, LW>(l, n, A, lda, min(i, rend - 1), t0 + H0, tb - H0, vec);
             }
         }
     }
