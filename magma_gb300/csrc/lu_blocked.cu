@@ -877,20 +877,33 @@ static magma_int_t blocked_getrf_outer(int m, int n, T **dA, int ldda, int **ipi
 // (step kernels / one CTA, us):
 //   FP64 n=64:  b=4 146 / 144, b=1000 279 / 281, b=3000 740 / 679
 //        n=80:  b=4 222 / 175, b=3000 1633 / 1258;  n=112: b=4 341 / 337, b=3000 4088 / 2797
-//        n=128: b=4 380 / 431, b=76 414 / 435, b=100 449 / 437, b=152 480 / 437, b=3000 4771 / 3965
-//        n=160: b=8 497 / 599, b=76 570 / 603, b=152 715 / 607, b=1500 4527 / 3867
-//        n=200: b=8 699 / 1035, b=76 996 / 1041, b=152 1389 / 1043, b=1500 9807 / 7347
-//        n=256: b=8 890 / 1875, b=76 1440 / 1885, b=152 2113 / 1903, b=1500 16641 / 15228
+//        n=128: b=4 380 / 431, b=76 414 / 435, b=100 449 / 437, b=152 480 / 437, b=153 580 / 566
+//        n=160: b=8 497 / 599, b=114 649 / 604, b=152 714 / 605, b=170 878 / 903, b=200 927 / 904
+//        n=200: b=8 699 / 1035, b=114 1191 / 1041, b=153 1538 / 1646, b=170 1618 / 1656, b=200 1755 / 1660
+//        n=215: b=153 1655 / 2056, b=200 1885 / 2072, b=228 2029 / 2078, b=310 2799 / 2957
+//        n=230: b=153 2152 / 2408, b=170 2276 / 2412, b=200 2508 / 2415, b=304 3342 / 2455
+//        n=256: b=8 890 / 1875, b=114 1788 / 1898, b=152 2111 / 1898, b=153 2392 / 3238, b=200 2775 / 3272,
+//               b=250 3222 / 3316, b=304 3701 / 3352, b=330 4330 / 4788, b=1500 16641 / 15228
 //   FP32 n=33:  b=4 54 / 44, b=3000 134 / 105;   n=48: b=4 60 / 52, b=3000 166 / 136
 //        n=52:  b=4 62 / 66, b=3000 175 / 191;   n=128: b=8 149 / 187, b=1500 531 / 651
-// FP64 is bound by its pipe, which the one-CTA kernel wastes less of once there is
-// about a matrix per SM.  FP32 is bound by the steps' latency, and a 32-column panel
-// of the step kernels has half as many steps outside it.
+// FP64 is bound by its pipe, which the one-CTA kernel wastes less of while every SM has
+// as many matrices as the others: its time grows by whole matrices per SM, the steps'
+// with the batch.  So it takes a batch that fills its last round of one matrix per SM
+// well enough; how well grows with n (a step's launches weigh less) and, from one
+// multiple of 32 to the next, as the steps' last panel and tiles fill up.  The line is
+// fitted to where the two cross for 46 orders from 113 to 256 and 40 batches up to 760 on
+// 152 SMs; above the first round the chosen side is at most 10 % slower than the other one
+// there (38 % with one CTA for every batch of three quarters of a matrix per SM or more).
+// FP32 is bound by the steps' latency, and a 32-column panel of the step kernels has half
+// as many steps outside it.
 template <typename T>
 static bool one_cta_per_matrix(int n, int batch)
 {
     if (sizeof(T) == 4) return n <= 48;
-    return n <= 112 || (n <= CTA_MAX_N && 4LL * batch >= 3LL * mlu_sm_count());
+    if (n <= 112 || n > CTA_MAX_N) return n <= 112;
+    const long long sms = mlu_sm_count(), rounds = (batch + sms - 1) / sms;
+    const int percent = 33 + 8 * (mlu_ceildiv(n, 32) - 6) + (n - 1) % 32;
+    return 100LL * batch >= max(percent, rounds == 1 ? 75 : 0) * rounds * sms;
 }
 
 // The kernels that a factorisation of `batch` matrices of order n launches under the
