@@ -749,12 +749,12 @@ magma_int_t magma_sposv_batched(magma_uplo_t uplo, magma_int_t n, magma_int_t nr
  * per-step kernels of the fixed-size path with per-matrix sizes (several CTAs
  * per matrix and step).
  *
- * magma_?getrf_vbatched_autotune: times the four choices that run different
- * code (panels of 8 or 16 columns, 4x4 or 2x2 elements) on `queue`'s device for
- * each bin up to max_n (bins above 256 are not timed), installs the fastest in
- * the table of that precision -- an installed entry that runs the same code as
- * the fastest stays as it is -- and returns the table in nb[8], tile[8] (either
- * may be NULL).  Allocates its trial
+ * magma_?getrf_vbatched_autotune: times 4x4 against 2x2 elements on panels of 16
+ * columns (and of 8 where that is installed) on `queue`'s device for each bin up
+ * to max_n (bins above 256 are not timed), installs the fastest in the table of
+ * that precision -- an installed entry that runs the same code as the fastest
+ * stays as it is -- and returns the table in nb[8], tile[8] (either may be NULL).
+ * Allocates its trial
  * batches and synchronises the queue.  max_n = 0 only returns the table.
  * Errors: -1 max_n < 0, -4 no queue, MAGMA_ERR_DEVICE_ALLOC.
  *

@@ -42,12 +42,14 @@ def test_autotuner_keeps_entries_that_no_candidate_reads(cuda, keep_tables, tile
     assert [v["band_ctas"] for v in t.values()][:3] == [4] * 3
 
 
-def test_vbatched_autotuner_times_only_different_kernels(cuda, keep_tables):
+@pytest.mark.parametrize("nb,candidates", [(32, 2), (16, 2), (8, 4)])
+def test_vbatched_autotuner_times_only_different_kernels(cuda, keep_tables, nb, candidates):
     lib = L.load()
     for dt in (torch.float64, torch.float32):
-        mg.set_vbatched_tuning([32] * 8, [1] * 8, dt)
+        mg.set_vbatched_tuning([nb] * 8, [1] * 8, dt)
         before = lib.magma_lu_launch_count()
         t = mg.autotune_vbatched(16, dt)
-        # the arrays, then widths 8 and 16 x tiles 4x4 and 2x2, twice each: fill, sort, factor
-        assert lib.magma_lu_launch_count() - before == 1 + 4 * 2 * 3
-        assert t["<=16"]["nb"] in (32, 8) and t["<=16"]["tile"] in (mg.batched.TILES[1], mg.batched.TILES[2])
+        # the arrays, then tiles 4x4 and 2x2 at width 16 (and the installed 8), twice each:
+        # fill, sort, factor
+        assert lib.magma_lu_launch_count() - before == 1 + candidates * 2 * 3
+        assert t["<=16"]["nb"] in (nb, 16) and t["<=16"]["tile"] in (mg.batched.TILES[1], mg.batched.TILES[2])
