@@ -1249,8 +1249,8 @@ TRAFFIC = {
                 "(profiles/ir_residual_kernel_fp64_n512_batch128.md)"},
     "gesv32": {
         "kernel": "mlu::small_gesv_packed_kernel<double>", "unit": "matrix (n=32, nrhs=1)",
-        "dram_bytes_per_unit": 110.8e6 / 10000,
-        "note": "ncu capture of one launch over 10,000 matrices: 84.9 MB read + 25.8 MB written "
+        "dram_bytes_per_unit": 110.3e6 / 10000,
+        "note": "ncu capture of one launch over 10,000 matrices: 84.7 MB read + 25.6 MB written "
                 "(profiles/small_gesv_kernel_fp64_n32_batch10000.md)"},
 }
 
