@@ -154,9 +154,9 @@ __device__ __forceinline__ T shfl(T v, int src) { return __shfl_sync(FULL, v, sr
 // Bounds-check build (-DMLU_BOUNDS_CHECK, the library's stand-in for a memory
 // sanitizer): MLU_BC2(r, c, m, n, site) is true when element (r, c) lies inside
 // the logical m x n operand; otherwise it records the first violation (site,
-// r, c) in a device word, counts it, and is false, so that the caller skips the
+// r, c) on the device, counts it, and is false, so that the caller skips the
 // access.  In the normal build it is the constant true and costs nothing.
-// Every translation unit has a record of its own (bc_record), which its object registers
+// Every translation unit has a record of its own (g_bc_record), which its object registers
 // with the reader (runtime.cu): so the build needs no relocatable device code and its
 // kernels are compiled as the normal library's are, but for the checks.
 #ifdef MLU_BOUNDS_CHECK
