@@ -20,8 +20,12 @@ namespace mlu {
 constexpr int GETRI_NR = 8;
 constexpr int GETRI_THREADS = 256;
 
-template <typename T>
-__global__ void __launch_bounds__(GETRI_THREADS, sizeof(T) == 8 ? 2 : 3)
+// CTAS: CTAs of 256 threads that the registers have to leave room for on an SM (0: as the
+// compiler likes).  FP32 has two forms: three CTAs (80 registers, with spills) where the
+// launch fills the SMs, 143 registers where it does not (n = 1000, one matrix 398 us with
+// three, 277 without; 20 matrices 3226 and 4637; n = 8, 3000 matrices 19.1 and 25.2).
+template <typename T, int CTAS>
+__global__ void __launch_bounds__(GETRI_THREADS, CTAS)
 getri_kernel(int n, T **dA_array, int ldda, int **ipiv_array, T **dInv_array, int lddia)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -62,8 +66,17 @@ static magma_int_t getri_run(const char *name, magma_int_t n, T **dA_array, magm
     }
     if (n == 0 || batchCount == 0) return 0;
     const size_t smem = (size_t)GETRI_NR * solve_ldx<T>(n) * sizeof(T);
-    static size_t dyn_cache[MLU_MAX_DEVICES];
-    const size_t dyn_max = mlu_device_cached(dyn_cache, [] { return mlu_allow_dynamic_smem(getri_kernel<T>); });
+    constexpr int FEW = sizeof(T) == 8 ? 2 : 0, MANY = sizeof(T) == 8 ? 2 : 3;
+    static size_t dyn_cache[MLU_MAX_DEVICES], sms_cache[MLU_MAX_DEVICES];
+    const size_t dyn_max = mlu_device_cached(dyn_cache, [] {
+        return min(mlu_allow_dynamic_smem(getri_kernel<T, FEW>), mlu_allow_dynamic_smem(getri_kernel<T, MANY>));
+    });
+    const size_t sms = mlu_device_cached(sms_cache, [] {
+        int dev = 0, count = 1;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+        return (size_t)max(count, 1);
+    });
     // the largest order: the right-hand sides and one int per row in shared memory
     const size_t limit = dyn_max + GETRI_NR * sizeof(int) + (sizeof(T) == 4 ? 128 + 32 * 3 * sizeof(T) : 0);
     if ((size_t)GETRI_NR * n * sizeof(T) + (size_t)n * sizeof(int) > limit || smem > dyn_max)
@@ -73,8 +86,13 @@ static magma_int_t getri_run(const char *name, magma_int_t n, T **dA_array, magm
     for (int b0 = 0; b0 < batchCount; b0 += MLU_MAX_GRID_Y) {
         const int nb = min(batchCount - b0, (int)MLU_MAX_GRID_Y);
         const dim3 grid((n + GETRI_NR - 1) / GETRI_NR, nb);
-        MLU_LAUNCH(mlu::KC_GETRS, s, getri_kernel<T><<<grid, threads, smem, s>>>(
-            n, dA_array + b0, ldda, dipiv_array + b0, dinvA_array + b0, lddia));
+        // (measured beside the kernel: from two CTAs of 256 threads per SM on)
+        if ((size_t)grid.x * nb * threads >= 2 * GETRI_THREADS * sms)
+            MLU_LAUNCH(mlu::KC_GETRS, s, getri_kernel<T, MANY><<<grid, threads, smem, s>>>(
+                n, dA_array + b0, ldda, dipiv_array + b0, dinvA_array + b0, lddia));
+        else
+            MLU_LAUNCH(mlu::KC_GETRS, s, getri_kernel<T, FEW><<<grid, threads, smem, s>>>(
+                n, dA_array + b0, ldda, dipiv_array + b0, dinvA_array + b0, lddia));
     }
     MLU_CHECK_LAUNCH();
     return 0;
